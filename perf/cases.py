@@ -212,9 +212,16 @@ def _lattice(case, seed):
 
 def _reference_start(case, seed):
     """Populations of a running reference-mode lattice: equilibrium of the flow, inside the
-    shaders' clamps (FP32, absolute, every cell)."""
-    rho, ux, uy = (t.double() for t in _flow(case, seed))
-    return torch.stack(_equilibrium(rho, ux, uy)).to(torch.float32)
+    shaders' clamps (FP32, absolute).  A wall holds what it hands back to a fluid cell inside
+    the outer ring, and nothing else."""
+    rho, ux, uy = (t.double() for t in _flow(dict(case, scene="channel"), seed))
+    f = torch.stack(_equilibrium(rho, ux, uy)).to(torch.float32)
+    solid, _ = _reference_mask(case["nx"], case["ny"], case["scene"])
+    takes = ~solid
+    takes[0], takes[-1], takes[:, 0], takes[:, -1] = (False,) * 4
+    for j in range(9):
+        f[j][solid & ~torch.roll(takes, (-EY[j], -EX[j]), (0, 1))] = 0.0
+    return f
 
 
 def _equilibrium(rho, ux, uy):
@@ -269,8 +276,7 @@ def prepare(case, seed):
         s["views"] = {"macro": _macro_views(sim)}
     elif kind == "frame":
         s["sim"] = sim = FluidSimulator(case["nx"], case["ny"], tau=0.62, pixel_size=2)
-        flow = dict(case, scene="channel")
-        sim.write_populations(_reference_start(flow, seed).cpu().numpy())
+        sim.write_populations(_reference_start(dict(case, scene="poiseuille"), seed).cpu().numpy())
         s["particles"] = p = Particles(sim, count=case["particles"], seed=seed)
         s["views"] = {"macro": _macro_views(sim), "rgba": _view(p, p.present(), (p.canvas_h, p.canvas_w, 4), "f32")}
     elif kind == "run":

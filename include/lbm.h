@@ -73,7 +73,9 @@ extern "C" {
 #define LBM_DTYPE_BF16 3 /* physics mode only: f_i - w_i in BF16, FP32 arithmetic */
 
 /* step kernel variants (physics mode) */
-#define LBM_KERNEL_AUTO 0   /* the fastest measured variant: LBM_KERNEL_CELL for FP32 / FP64;
+#define LBM_KERNEL_AUTO 0   /* the fastest measured variant: LBM_KERNEL_CELL for FP32 / FP64 (FP32 BGK
+                               and KBC lattices of 800,000 cells or more take up to three steps per
+                               launch, with the results of single steps bit for bit);
                                for FP16 / BF16 LBM_KERNEL_TILED where it applies, else
                                LBM_KERNEL_VEC2 (nx even) */
 #define LBM_KERNEL_CELL 1   /* one cell per thread */

@@ -103,6 +103,7 @@ void pool_free(void* p, cudaStream_t s) {
 }
 
 constexpr float OBSTACLE_RADIUS = 28.0f;  // fluid/mod.rs:1
+constexpr int FORCE_STEPS = 90;           // steps a force stroke's cells act (d2q9_node.rs:263-300)
 
 bool sd_sphere(float px, float py, float r) {  // fluid/mod.rs:57-59 (glam Vec2::length)
     const float d = std::sqrt(px * px + py * py);
@@ -337,7 +338,7 @@ lbm_lattice_info force_stroke(int nx, int ny, int pixel_size, float pos_x, float
         if (x < 1 || (long)x >= (long)nx - 2 || y < 1 || (long)y >= (long)ny - 2) continue;
         cells.push_back((size_t)y * nx + x);
     }
-    return make_info(LBM_EXTERNAL_FORCE, vx, vy, 90);
+    return make_info(LBM_EXTERNAL_FORCE, vx, vy, FORCE_STEPS);
 }
 
 int validate_params(const lbm_params& p) {
@@ -426,6 +427,7 @@ int scene_and_state_on_device(lbm_handle* h) {
     }
     h->host_info.clear();
     h->host_info_lazy = true;
+    h->no_solids = h->p.scene == LBM_SCENE_PERIODIC;
     return LBM_OK;
 }
 
@@ -454,7 +456,32 @@ int init_state(lbm_handle* h) {
     }
     ++h->launches;
     h->cur = 0;
+    h->solids_agree = true;  // zero in both buffers
     h->stepped_since_init = false;
+    return LBM_OK;
+}
+
+// the steps for which one of `count` records may still count down (k_ref_step, phys_collide:
+// block_iter of inlet and forcing cells)
+int64_t longest_countdown(const lbm_lattice_info* info, size_t count) {
+    int64_t n = 0;
+    for (size_t i = 0; i < count; ++i)
+        if (info[i].block_iter > 0 && (info[i].material == LBM_INLET || info[i].material == LBM_EXTERNAL_FORCE))
+            n = std::max<int64_t>(n, info[i].block_iter);
+    return n;
+}
+// an obstacle's upload brings back rows [y0, y1) of the host copy
+void restart_countdown(lbm_handle* h, int y0, int y1) {
+    const lbm_lattice_info* rows = h->host_info.data() + (size_t)y0 * h->nx;
+    h->countdown = std::max(h->countdown, longest_countdown(rows, (size_t)(y1 - y0) * h->nx));
+}
+// the same over the device's records, which were all replaced; waits for the stream
+int whole_countdown(lbm_handle* h) {
+    unsigned long long n = 0;
+    LBM_CK(lbm::launch_longest_countdown(h, h->stream));
+    LBM_CK(cudaMemcpyAsync(&n, h->d_count, sizeof(n), cudaMemcpyDeviceToHost, h->stream));
+    LBM_CK(cudaStreamSynchronize(h->stream));
+    h->countdown = (int64_t)n;
     return LBM_OK;
 }
 
@@ -657,11 +684,14 @@ int lbm_step(lbm_handle* h, int32_t nsteps) {
     LBM_TRY(check_handle(h));
     if (nsteps < 0) return fail(LBM_ERR_ARG, "negative step count");
     LBM_TRY(use_device(h));
-    for (int32_t s = 0; s < nsteps; ++s) {
-        const bool macro = h->p.macro_every_step || s == nsteps - 1;
-        LBM_CK(lbm::launch_step(h, macro, h->stream));
+    for (int32_t s = 0; s < nsteps;) {
+        const int n = lbm::fused_steps(h, nsteps - s);
+        const bool macro = h->p.macro_every_step || s + n == nsteps;
+        LBM_CK(n > 1 ? lbm::launch_fused(h, n, macro, h->stream) : lbm::launch_step(h, macro, h->stream));
+        s += n;
         h->cur ^= 1;
-        ++h->steps;
+        h->steps += n;
+        h->countdown = std::max<int64_t>(0, h->countdown - n);
         ++h->launches;
     }
     if (nsteps > 0) h->stepped_since_init = true;
@@ -688,6 +718,8 @@ int lbm_reset(lbm_handle* h) {
         if (r == LBM_OK) r = init_state(h);
     }
     if (r == LBM_OK) r = rebuild_flags(h);
+    // no record counts down: a new scene has permanent ones only, and init.wgsl ends the others
+    if (r == LBM_OK) h->countdown = 0;
     h->pre_x = h->pre_y = 0.0f;  // fluid_simulator.rs:214
     const int rs = sync(h);      // also before the disk list is released on a failed launch
     h->scene_disks = std::vector<double>();
@@ -716,6 +748,8 @@ int lbm_add_obstacle(lbm_handle* h, int32_t x, int32_t y) {
         return fail(LBM_ERR_ARG, "obstacle rows [%d, %d) or column %d outside the lattice", min_y, max_y, x);
     LBM_TRY(use_device(h));
     ensure_host_info(h);
+    h->no_solids = h->solids_agree = false;
+    restart_countdown(h, min_y, max_y);
     obstacle_disc(h->nx, x, y, h->host_info.data());
     // the reference uploads whole rows from its host copy (d2q9_node.rs:243-244)
     LBM_TRY(upload_info_rows(h, min_y, max_y));
@@ -764,6 +798,7 @@ int lbm_add_external_force(lbm_handle* h, float pos_x, float pos_y, float pre_x,
     if (h->p.pixel_size < 2)
         return fail(LBM_ERR_ARG, "force strokes need pixel_size >= 2 (the reference divides by pixel_size - 1)");
     LBM_TRY(use_device(h));
+    h->countdown = std::max<int64_t>(h->countdown, FORCE_STEPS);
     std::vector<size_t> cells;
     const lbm_lattice_info rec = force_stroke(h->nx, h->ny, h->p.pixel_size, pos_x, pos_y, pre_x, pre_y, cells);
     // queue.write_buffer of one record per cell; the host copy is not updated, as in the reference
@@ -883,6 +918,11 @@ int lbm_apply_edits(lbm_handle* h, const lbm_edit* edits, int32_t n, int32_t* ap
         const auto* d_obs = (const lbm::EditObstacle*)h->d_edits;
         const auto* d_forces = (const lbm::EditForce*)((const unsigned char*)h->d_edits +
                                                         obs.size() * sizeof(lbm::EditObstacle));
+        if (!obs.empty()) {
+            h->no_solids = h->solids_agree = false;
+            restart_countdown(h, row0, row1);
+        }
+        if (!forces.empty()) h->countdown = std::max<int64_t>(h->countdown, FORCE_STEPS);
         LBM_CK(lbm::launch_edits(h, d_obs, (int)obs.size(), d_forces, (int)forces.size(), row0, row1, h->stream));
         h->launches += (obs.empty() ? 0 : 1) + (forces.empty() ? 0 : 1);
         LBM_TRY(rebuild_flags(h));
@@ -939,9 +979,12 @@ int lbm_set_info(lbm_handle* h, const lbm_lattice_info* info) {
     LBM_TRY(use_device(h));
     h->host_info.assign(info, info + h->N);
     h->host_info_lazy = false;
+    h->no_solids = false;
+    h->solids_agree = false;  // a new solid cell keeps what it held as fluid, another step in each buffer
+    h->countdown = INT64_MAX;
     LBM_TRY(upload_info_rows(h, 0, h->ny));
     LBM_TRY(rebuild_flags(h));
-    return sync(h);
+    return whole_countdown(h);
 }
 
 int lbm_get_info(lbm_handle* h, lbm_lattice_info* out) {
@@ -1010,9 +1053,14 @@ int lbm_write_populations(lbm_handle* h, const void* src, int32_t sd) {
     cudaError_t e = cudaMemcpyAsync(tmp, src, bytes, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) e = lbm::launch_from_absolute(h, tmp, sd, h->buf[h->cur], h->stream);
     pool_free(tmp, h->stream);
+    h->solids_agree = false;
+    unsigned long long differ = 1;
+    if (e == cudaSuccess) e = lbm::launch_count_solid_slots(h, h->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&differ, h->d_count, sizeof(differ), cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "population upload: %s", cudaGetErrorString(e));
-    ++h->launches;
+    h->solids_agree = differ == 0;
+    h->launches += 2;
     return LBM_OK;
 }
 
@@ -1037,6 +1085,7 @@ int lbm_init_equilibrium(lbm_handle* h, const float* rho, const float* ux, const
     if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "equilibrium initialisation: %s", cudaGetErrorString(e));
     ++h->launches;
     h->cur = 0;
+    h->solids_agree = true;  // zero in both buffers
     h->stepped_since_init = false;
     return LBM_OK;
 }
@@ -1166,6 +1215,8 @@ int lbm_load(lbm_handle* h, const char* path) {
     h->host_info = hinfo;
     h->host_info_lazy = false;
     h->host_mirror_valid = false;
+    h->countdown = INT64_MAX;
+    h->no_solids = h->solids_agree = false;
     h->cur = hd.cur & 1;
     h->tau = hd.tau;
     h->omega = 1.0f / hd.tau;
@@ -1177,7 +1228,7 @@ int lbm_load(lbm_handle* h, const char* path) {
     h->p.scene = hd.scene;
     h->fluid_ty = hd.fluid_ty;
     LBM_TRY(rebuild_flags(h));
-    return sync(h);
+    return whole_countdown(h);
 }
 
 int lbm_status(lbm_handle* h) {
@@ -1214,7 +1265,7 @@ int lbm_bounds_report(uint64_t* count, uint64_t* first_index, uint64_t* first_li
 #ifdef LBM_BOUNDS_CHECK
     lbm::BoundsRecord total{};
     cudaError_t (*takes[])(lbm::BoundsRecord*) = {lbm::bounds_take_kernels, lbm::bounds_take_vec,
-                                                 lbm::bounds_take_bulk, lbm::bounds_take_batch};
+                                                 lbm::bounds_take_bulk, lbm::bounds_take_batch, lbm::bounds_take_fused};
     for (auto take : takes) {
         lbm::BoundsRecord r{};
         LBM_CK(take(&r));

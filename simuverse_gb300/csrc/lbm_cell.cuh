@@ -10,6 +10,7 @@
 #pragma once
 
 #include "lbm_common.cuh"
+#include "lbm_core.cuh"
 
 namespace lbm {
 
@@ -345,7 +346,10 @@ __device__ __forceinline__ void phys_cell_update(const typename ST::T* __restric
         }
     }
     R o[9], rho, ux, uy;
-    phys_collide<R, COLL>(d, m, fl, (size_t)cc, flags, info, omega, o, rho, ux, uy, R(ST::UNIT));
+    if constexpr (core_has(COLL) && ST::dtype == LBM_DTYPE_F32)
+        core_cell<R, COLL>(d, m, fl, (size_t)cc, flags, info, omega, o, rho, ux, uy);
+    else
+        phys_collide<R, COLL>(d, m, fl, (size_t)cc, flags, info, omega, o, rho, ux, uy, R(ST::UNIT));
     if (MACRO && in_bounds(mc + 2 * N, end_m, BS_CELL_MACRO)) {
         macro[mc] = (float)rho; macro[mc + N] = (float)ux; macro[mc + 2 * N] = (float)uy;
     }

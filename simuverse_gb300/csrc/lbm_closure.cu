@@ -899,6 +899,7 @@ int lbm_coarsen(lbm_handle* fine, lbm_handle* coarse, int32_t factor, float neq_
                                                     neq_scale, (float*)coarse->buf[coarse->cur]);
     C_CK(cudaGetLastError());
     coarse->launches += 1;
+    coarse->solids_agree = false;  // every cell of the current buffer was written
     C_CK(cudaStreamSynchronize(coarse->stream));
     return LBM_OK;
 }
@@ -996,6 +997,7 @@ int lbm_closure_apply(lbm_closure* c, lbm_handle* h) {
     C_TRY(check_coarse(c, h));
     C_CK(cudaSetDevice(c->device));
     const int r = correction(c, h, (float*)h->buf[h->cur], 1);
+    h->solids_agree = false;  // solid cells of one buffer were written too
     if (c->kernel == LBM_CLOSURE_KERNEL_FUSED)  // one kernel, plus the field means and the apply pass
         h->launches += c->projection == LBM_CLOSURE_PROJECT_DOMAIN ? 4 : (c->target == LBM_CLOSURE_TARGET_STRESS ? 2 : 1);
     else

@@ -78,6 +78,7 @@ enum BoundsSite : int {
     BS_CELL_FLAGS = 11, BS_CELL_PULL, BS_CELL_INFO, BS_CELL_STORE, BS_CELL_MACRO,
     BS_TILE_FLAGS = 21, BS_TILE_PULL, BS_TILE_INFO, BS_TILE_STORE, BS_TILE_MACRO,
     BS_BULK_COPY = 31, BS_BULK_PULL, BS_BULK_INFO, BS_BULK_STORE, BS_BULK_MACRO,
+    BS_FUSED_FLAGS = 41, BS_FUSED_PULL, BS_FUSED_INFO, BS_FUSED_STORE, BS_FUSED_MACRO,
     BS_SELFTEST = 99
 };
 #ifdef LBM_BOUNDS_CHECK

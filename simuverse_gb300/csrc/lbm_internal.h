@@ -51,6 +51,11 @@ struct lbm_handle {
     cudaStream_t own_stream = nullptr;
     uint64_t steps = 0;
     uint64_t launches = 0;
+    // what the fused steps (lbm_step_fused.cu) ask: steps for which a forcing cell's record may still
+    // count down; a lattice without any solid cell; whether the solid cells' slots that no step
+    // writes hold the same in both buffers
+    int64_t countdown = 0;
+    bool no_solids = false, solids_agree = false;
     bool stepped_since_init = false;  // macro_tex holds (0,0,0,1) right after init
     float pre_x = 0.0f, pre_y = 0.0f;  // FluidSimulator::pre_pos
     int device = 0;
@@ -111,6 +116,7 @@ cudaError_t bounds_take_kernels(BoundsRecord* out);  // lbm_kernels.cu: k_ref_st
 cudaError_t bounds_take_vec(BoundsRecord* out);      // lbm_step_vec.cu: k_phys_step_tiled
 cudaError_t bounds_take_bulk(BoundsRecord* out);     // lbm_step_bulk.cu: k_phys_step_bulk
 cudaError_t bounds_take_batch(BoundsRecord* out);    // lbm_batch.cu: the batched one-cell update
+cudaError_t bounds_take_fused(BoundsRecord* out);    // lbm_step_fused.cu: the fused steps
 // one thread evaluates one index equal to its extent (no memory access): the record must show it
 cudaError_t bounds_selftest(cudaStream_t s);
 #endif
@@ -136,6 +142,13 @@ cudaError_t launch_ref_init(lbm_handle* h, cudaStream_t s);
 cudaError_t launch_phys_init(lbm_handle* h, const float* d_rho, const float* d_ux, const float* d_uy,
                              cudaStream_t s);
 cudaError_t launch_step(lbm_handle* h, bool write_macro, cudaStream_t s);
+// fused steps (lbm_step_fused.cu): how many of the next `left` steps one launch takes (1: launch_step)
+int fused_steps(const lbm_handle* h, int left);
+cudaError_t launch_fused(lbm_handle* h, int steps, bool write_macro, cudaStream_t s);
+// *d_count (of h) = largest block_iter of an inlet or forcing cell's record, 0 without a positive one
+cudaError_t launch_longest_countdown(lbm_handle* h, cudaStream_t s);
+// *d_count (of h) = solid cells' slots that no step writes and that differ between the buffers
+cudaError_t launch_count_solid_slots(lbm_handle* h, cudaStream_t s);
 // four-cells-per-thread physics step (lbm_step_vec.cu)
 bool vec_step_supported(const lbm_handle* h);
 cudaError_t launch_phys_step_vec(lbm_handle* h, bool write_macro, cudaStream_t s);

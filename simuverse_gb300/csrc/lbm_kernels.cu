@@ -499,6 +499,50 @@ __global__ void k_count_nonfinite(const typename ST::T* __restrict__ A, size_t t
     if ((threadIdx.x & 31) == 0 && local) atomicAdd(count, local);
 }
 
+__global__ void __launch_bounds__(RED_TPB) k_longest_countdown(const lbm_lattice_info* __restrict__ info, size_t N,
+                                                               unsigned long long* longest) {
+    unsigned n = 0;
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < N; c += stride) {
+        const int2 r = *reinterpret_cast<const int2*>(info + c);  // material, block_iter
+        if (r.y > 0 && (r.x == LBM_INLET || r.x == LBM_EXTERNAL_FORCE)) n = max(n, (unsigned)r.y);
+    }
+    n = __reduce_max_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31) == 0 && n) atomicMax(longest, (unsigned long long)n);
+}
+
+// slots of solid cells that no step writes and whose bits differ between the buffers.  Physics
+// mode: all nine.  Reference mode: not those it zeroes (wall-to-wall) and not those a fluid cell
+// strictly inside the outer ring hands its population to.
+__global__ void __launch_bounds__(RED_TPB) k_count_solid_slots(const unsigned char* __restrict__ A,
+                                                               const unsigned char* __restrict__ B, int elem_bytes,
+                                                               const uint16_t* __restrict__ flags, int nx, int ny,
+                                                               int mode, bool tiled, unsigned long long* count) {
+    unsigned long long local = 0;
+    const size_t N = (size_t)nx * ny, stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < N; c += stride) {
+        const unsigned fl = flags[c];
+        if (!is_solid((int)(fl & FL_MAT_MASK))) continue;
+        const int x = (int)(c % (size_t)nx), y = (int)(c / (size_t)nx);
+        for (int j = 0; j < 9; ++j) {
+            if (mode == LBM_MODE_REFERENCE) {
+                const int px = x + EX(j), py = y + EY(j);
+                if (fl & (1u << (FL_DIR_SHIFT + j))) continue;
+                if (px > 0 && py > 0 && px < nx - 1 && py < ny - 1 &&
+                    !is_solid((int)(flags[(size_t)py * nx + px] & FL_MAT_MASK)))
+                    continue;
+            }
+            const size_t b = pop_index(tiled, N, j, c) * (size_t)elem_bytes;
+            bool same = true;
+            for (int k = 0; k < elem_bytes; k += 2)
+                same &= *reinterpret_cast<const uint16_t*>(A + b + k) == *reinterpret_cast<const uint16_t*>(B + b + k);
+            if (!same) ++local;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) local += __shfl_down_sync(0xffffffffu, local, o);
+    if ((threadIdx.x & 31) == 0 && local) atomicAdd(count, local);
+}
+
 // sums over non-solid cells of h: |drho|^2, |rho_ref|^2, |du|^2, |u_ref|^2, then maxima
 __global__ void __launch_bounds__(RED_TPB) k_macro_error(const float* __restrict__ m, const float* __restrict__ mref,
                                                          const uint16_t* __restrict__ flags, size_t N,
@@ -815,6 +859,22 @@ cudaError_t launch_count_nonfinite(lbm_handle* h, cudaStream_t s) {
         case LBM_DTYPE_F16: k_count_nonfinite<StoreF16><<<RED_BLOCKS, RED_TPB, 0, s>>>((const __half*)h->buf[h->cur], total, h->d_count); break;
         default: k_count_nonfinite<StoreBF16><<<RED_BLOCKS, RED_TPB, 0, s>>>((const __nv_bfloat16*)h->buf[h->cur], total, h->d_count); break;
     }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_longest_countdown(lbm_handle* h, cudaStream_t s) {
+    const cudaError_t e = cudaMemsetAsync(h->d_count, 0, sizeof(unsigned long long), s);
+    if (e != cudaSuccess) return e;
+    k_longest_countdown<<<RED_BLOCKS, RED_TPB, 0, s>>>(h->d_info, h->N, h->d_count);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_count_solid_slots(lbm_handle* h, cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(h->d_count, 0, sizeof(unsigned long long), s);
+    if (e != cudaSuccess) return e;
+    k_count_solid_slots<<<RED_BLOCKS, RED_TPB, 0, s>>>((const unsigned char*)h->buf[0], (const unsigned char*)h->buf[1],
+                                                       (int)dtype_size(h->p.dtype), h->d_flags, h->nx, h->ny,
+                                                       h->p.mode, h->tiled, h->d_count);
     return cudaGetLastError();
 }
 

@@ -11,8 +11,9 @@
 // into runs of tx * ty consecutive cells of the padded rows, which leave no partly filled
 // tile at a domain's right edge; a tile list covers them all (one cell per thread, or four
 // with vector accesses).
-// Method 0: one cooperative persistent launch runs every step: blocks take tiles
-// round-robin, then meet at a grid barrier before the next step.  The barrier spins with
+// Method 0: one cooperative persistent launch runs every step: warps take windows of a domain for
+// up to three fused steps (k_batch_march), or, where a domain is too small for them, blocks take tiles
+// round-robin for one step; then they meet at a grid barrier.  The barrier spins with
 // a time limit: a block that waits longer sets an error word (LBM_ERR_TIMEOUT), every
 // waiting block sees it and leaves, and the host reads the status -- no trap, the context
 // stays usable.  The launch (with the barrier reset) is captured once into a CUDA graph
@@ -36,6 +37,7 @@
 #include "lbm_cell4.cuh"
 #include "lbm_common.cuh"
 #include "lbm_internal.h"
+#include "lbm_march.cuh"
 
 namespace lbm {
 
@@ -52,6 +54,7 @@ struct BarrierState {
     int error;
     int where_step;
     int where_block;
+    unsigned int ticket[3];  // k_batch_march: next task of a pass, by pass number mod 3
 };
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -180,6 +183,68 @@ __global__ void __launch_bounds__(256, batch_min_blocks(KF)) k_batch_persistent(
         if (!grid_barrier(bar, (unsigned)(s + 1) * gridDim.x, timeout_ns, s)) return;
     }
 }
+// method 0 for batches whose domains are wide and tall enough: passes of up to three fused steps
+// (lbm_march.cuh).  A warp takes windows of 60 columns x some rows of a domain from a common counter,
+// since those at walls, inlets and outflows take longer (124 and 91 GLUPS where every window is one of
+// them, 180 inside); the blocks meet at the grid barrier once per pass.  One step per pass moves 74 bytes
+// per cell and ran at 86 % of the measured copy bandwidth; three move about 26.  256 domains of 64 to
+// 1024 cells a side: 80 -> 117 GLUPS, 64 domains 77 -> 89 (what bounds those: two to three tasks per
+// warp and pass, uneven ones, and windows that a domain's width fills badly).
+// the last pass of a call that is no multiple of three steps: a function, which costs the loop nothing
+template <int T>
+__device__ __noinline__ void march_rest(const FusedLattice& L, const BgkConst<float2>& k, int x0, int y0, int y1, bool macro,
+                                        uint32_t smem) {
+    march_window<T, LBM_COLLISION_BGK, true>(L, k, x0, y0, y1, macro, smem);
+}
+constexpr int BM_WARPS = 4;   // warps of a block, each on its own
+constexpr int BM_BLOCKS = 3;  // blocks per SM the kernel is compiled for: 168 registers, no spills
+__global__ void __launch_bounds__(32 * BM_WARPS, BM_BLOCKS)
+    k_batch_march(const BatchDomain* __restrict__ doms, const int4* __restrict__ tasks, int ntasks, float* pool0,
+                  float* pool1, const uint16_t* flags, const lbm_lattice_info* info, float* macro, int nsteps, int cur0,
+                  bool write_macro, BarrierState* bar, unsigned long long timeout_ns, int skip_block, int skip_step) {
+    extern __shared__ __align__(16) unsigned char march_mem[];
+    __shared__ FusedLattice lattices[BM_WARPS];
+    const int wid = (int)threadIdx.x >> 5;
+    const uint32_t smem = (uint32_t)__cvta_generic_to_shared(march_mem) + (uint32_t)(wid * MARCH_SMEM);
+    const int warps = (int)gridDim.x * BM_WARPS;
+    for (int done = 0, pass = 0; done < nsteps; ++pass) {
+        const int left = nsteps - done, T = left == 4 ? 2 : min(left, 3);
+        const bool odd = ((cur0 + pass) & 1) != 0, mac = write_macro && left == T;
+        if (blockIdx.x == 0 && threadIdx.x == 0) bar->ticket[(pass + 1) % 3] = 0;  // the next pass's, last used two passes ago
+        int t = (int)blockIdx.x * BM_WARPS + wid;
+        while (t < ntasks) {
+            unsigned next = 0;  // asked for before the task, needed after it
+            if ((threadIdx.x & 31) == 0) next = atomicAdd(&bar->ticket[pass % 3], 1u);
+            const int4 q = tasks[t];
+            const BatchDomain dm = doms[q.x];
+            // in shared memory: the march reads its pointers there, it has no registers for them
+            FusedLattice& L = lattices[wid];
+            __syncwarp();
+            if ((threadIdx.x & 31) == 0) {
+                L.A = (odd ? pool1 : pool0) + dm.pop_off;
+                L.B = (odd ? pool0 : pool1) + dm.pop_off;
+                L.flags = flags + dm.cell_off;
+                L.info = info + dm.cell_off;
+                L.macro = macro + 3 * dm.cell_off;
+                L.nx = dm.nx;
+                L.pitch = dm.pitch;
+                L.ny = dm.ny;
+                L.N = (uint32_t)(dm.pitch * dm.ny);
+            }
+            __syncwarp();
+            const BgkConst<float2> k(dm.omega);
+            if (T == 3) march_window<3, LBM_COLLISION_BGK, true>(L, k, q.y, q.z, q.w, mac, smem);
+            else if (T == 2) march_rest<2>(L, k, q.y, q.z, q.w, mac, smem);
+            else march_rest<1>(L, k, q.y, q.z, q.w, mac, smem);
+            t = warps + (int)__shfl_sync(0xffffffffu, next, 0);
+        }
+        if ((int)blockIdx.x == skip_block && skip_step >= done && skip_step < done + T) return;  // injected (tests)
+        if (!grid_barrier(bar, (unsigned)(pass + 1) * gridDim.x, timeout_ns, done + T - 1)) return;
+        done += T;
+    }
+}
+// the passes of nsteps steps (the kernel's split)
+static inline int march_passes(int nsteps) { return (nsteps + 2) / 3; }
 // method 1: one step over the tile list, one tile per block
 template <int KF>
 __global__ void __launch_bounds__(256, batch_min_blocks(KF)) k_batch_tiles(const BatchDomain* __restrict__ doms, const int4* __restrict__ tiles,
@@ -305,7 +370,11 @@ struct TuneKey {
     int ndom;
     bool operator<(const TuneKey& o) const { return std::tie(cells_class, ndom) < std::tie(o.cells_class, o.ndom); }
 };
-std::map<TuneKey, lbm_batch_config> g_tune_cache;
+struct Tuned {
+    lbm_batch_config cfg;
+    int rows;  // of a task of k_batch_march, 0 where it does not apply
+};
+std::map<TuneKey, Tuned> g_tune_cache;
 
 }  // namespace
 
@@ -315,6 +384,9 @@ struct lbm_batch {
     lbm::BatchDomain* d_doms = nullptr;
     int4* d_tiles = nullptr;
     int ntiles = 0;
+    bool march = false;  // every domain fits the windows of k_batch_march
+    int4* d_tasks = nullptr;
+    int ntasks = 0, march_rows = 0;
     float* pool[2] = {nullptr, nullptr};
     uint16_t* d_flags = nullptr;
     lbm_lattice_info* d_info = nullptr;
@@ -363,6 +435,34 @@ int build_tiles(lbm_batch* b) {
     return LBM_OK;
 }
 
+// Tasks of k_batch_march: windows of MARCH_OUT columns x rows.  The first and last windows of a domain,
+// which hold its inlet, outflow or side walls, come first.
+std::vector<int4> march_tasks(const lbm_batch* b, int rows) {
+    std::vector<int4> edge, inner;
+    for (size_t d = 0; d < b->doms.size(); ++d) {
+        const lbm::BatchDomain& dm = b->doms[d];
+        for (int y0 = 0; y0 < dm.ny; y0 += rows)
+            for (int x0 = 0; x0 < dm.nx; x0 += lbm::MARCH_OUT)
+                (x0 == 0 || x0 + lbm::MARCH_OUT >= dm.nx ? edge : inner)
+                    .push_back(make_int4((int)d, x0, y0, std::min(y0 + rows, dm.ny)));
+    }
+    edge.insert(edge.end(), inner.begin(), inner.end());
+    return edge;
+}
+int set_march_rows(lbm_batch* b, int rows) {
+    if (rows == b->march_rows) return LBM_OK;
+    const std::vector<int4> tasks = march_tasks(b, rows);
+    if (b->d_tasks) cudaFree(b->d_tasks);
+    b->d_tasks = nullptr;
+    b->march_rows = 0;
+    free_graph(b);
+    B_CK(cudaMalloc((void**)&b->d_tasks, tasks.size() * sizeof(int4)));
+    B_CK(cudaMemcpy(b->d_tasks, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    b->ntasks = (int)tasks.size();
+    b->march_rows = rows;
+    return LBM_OK;
+}
+
 // the kernels' form KF (k_batch_persistent): tile form + 10 for the 32-register budget
 int tile_form(const lbm_batch* b) {
     const int f = b->cfg.linear ? 0 : b->cfg.cells_per_thread;
@@ -381,9 +481,41 @@ int with_form(const lbm_batch* b, F&& fn) {
     }
 }
 
+// Rows of a task: whole waves of warps with little work done twice (T - 1 rows above and below a task
+// are computed for its first steps): the rows that minimise waves x (rows + halo).
+int march_rows_for(const lbm_batch* b) {
+    const long warps = (long)b->sms * lbm::BM_BLOCKS * lbm::BM_WARPS;
+    long best = -1;
+    int rows = 0;
+    for (int r = 12; r <= 96; ++r) {
+        long tasks = 0;
+        for (const lbm::BatchDomain& dm : b->doms)
+            tasks += (long)((dm.nx + lbm::MARCH_OUT - 1) / lbm::MARCH_OUT) * ((dm.ny + r - 1) / r);
+        const long cost = (tasks + warps - 1) / warps * (r + 5);
+        if (best < 0 || cost < best) {
+            best = cost;
+            rows = r;
+        }
+    }
+    return rows;
+}
+
 int persistent_grid(lbm_batch* b, int* grid) {
     int per_sm = 0;
-    const int threads = b->cfg.tile_threads_x * b->cfg.tile_rows;
+    const int threads = b->march ? 32 * lbm::BM_WARPS : b->cfg.tile_threads_x * b->cfg.tile_rows;
+    if (b->march) {
+        constexpr int SMEM = lbm::BM_WARPS * lbm::MARCH_SMEM;
+        static lbm::PerDevice<int> fit;
+        B_CK(fit.get(
+            b->device,
+            [](int& n) {
+                const cudaError_t e = cudaFuncSetAttribute(lbm::k_batch_march, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+                return e != cudaSuccess ? e
+                                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, lbm::k_batch_march,
+                                                                                        32 * lbm::BM_WARPS, SMEM);
+            },
+            &per_sm));
+    } else
     B_TRY(with_form(b, [&](auto kf) {
         B_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lbm::k_batch_persistent<decltype(kf)::value>,
                                                            threads, 0));
@@ -395,20 +527,28 @@ int persistent_grid(lbm_batch* b, int* grid) {
     return LBM_OK;
 }
 
-int launch_persistent(lbm_batch* b, int nsteps, int skip_block, int skip_step, cudaStream_t s) {
+int launch_persistent(lbm_batch* b, int nsteps, int skip_block, int skip_step, cudaStream_t s, bool macro = true) {
     int grid = 0;
     B_TRY(persistent_grid(b, &grid));
     B_CK(cudaMemsetAsync(b->d_bar, 0, sizeof(lbm::BarrierState), s));
     cudaLaunchConfig_t lc;
     std::memset(&lc, 0, sizeof(lc));
     lc.gridDim = dim3((unsigned)grid);
-    lc.blockDim = dim3((unsigned)b->cfg.tile_threads_x, (unsigned)b->cfg.tile_rows);
+    lc.blockDim = b->march ? dim3(32u * lbm::BM_WARPS) : dim3((unsigned)b->cfg.tile_threads_x, (unsigned)b->cfg.tile_rows);
+    lc.dynamicSmemBytes = b->march ? lbm::BM_WARPS * lbm::MARCH_SMEM : 0;
     lc.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     lc.attrs = attr;
     lc.numAttrs = 1;
+    if (b->march) {
+        B_CK(cudaLaunchKernelEx(&lc, lbm::k_batch_march, (const lbm::BatchDomain*)b->d_doms, (const int4*)b->d_tasks,
+                                b->ntasks, b->pool[0], b->pool[1], (const uint16_t*)b->d_flags,
+                                (const lbm_lattice_info*)b->d_info, b->d_macro, nsteps, b->cur, macro, b->d_bar,
+                                b->timeout_ns, skip_block, skip_step));
+        return LBM_OK;
+    }
     B_TRY(with_form(b, [&](auto kf) {
         B_CK(cudaLaunchKernelEx(&lc, lbm::k_batch_persistent<decltype(kf)::value>, (const lbm::BatchDomain*)b->d_doms,
                                 (const int4*)b->d_tiles, b->ntiles, b->pool[0], b->pool[1], b->d_flags, b->d_info,
@@ -476,7 +616,8 @@ int run_steps(lbm_batch* b, int nsteps, int method) {
         }
         b->launches += (uint64_t)nsteps * b->doms.size();
     }
-    b->cur = (b->cur + nsteps) & 1;
+    // a pass of fused steps swaps the pools once (their solid and padding cells hold zeros in both)
+    b->cur = (b->cur + (method == LBM_BATCH_PERSISTENT && b->march ? lbm::march_passes(nsteps) : nsteps)) & 1;
     b->steps += nsteps;
     return LBM_OK;
 }
@@ -603,7 +744,10 @@ int lbm_batch_create(int32_t n, const lbm_domain_desc* desc, lbm_batch** out) {
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    b->march = true;
+    for (const lbm::BatchDomain& dm : doms) b->march = b->march && dm.nx >= lbm::MARCH_W && dm.ny >= 8;
     int r = e == cudaSuccess ? build_tiles(b) : bfail(LBM_ERR_CUDA, "batch set-up: %s", cudaGetErrorString(e));
+    if (r == LBM_OK && b->march) r = set_march_rows(b, march_rows_for(b));
     if (r != LBM_OK) {
         lbm_batch_destroy(b);
         return r;
@@ -626,6 +770,7 @@ int lbm_batch_destroy(lbm_batch* b) {
     cudaFree(b->d_bar);
     cudaFree(b->d_doms);
     cudaFree(b->d_tiles);
+    cudaFree(b->d_tasks);
     if (b->own_stream) cudaStreamDestroy(b->own_stream);
     delete b;
     return LBM_OK;
@@ -713,10 +858,23 @@ int lbm_batch_tune(lbm_batch* b, int32_t trial_steps, lbm_batch_config* best_out
     const TuneKey key{(long)std::lround(std::log2((double)b->live_cells + 1.0) * 4.0), (int)b->doms.size()};
     auto it = g_tune_cache.find(key);
     if (it != g_tune_cache.end()) {
-        B_TRY(lbm_batch_set_config(b, &it->second));
-        if (best_out) *best_out = it->second;
+        B_TRY(lbm_batch_set_config(b, &it->second.cfg));
+        if (b->march) B_TRY(set_march_rows(b, it->second.rows));
+        if (best_out) *best_out = it->second.cfg;
         return LBM_OK;
     }
+    // the tile shapes first (they serve the other methods, and this one where k_batch_march cannot)
+    const bool march = b->march;
+    b->march = false;
+    struct Restore {
+        lbm_batch* b;
+        bool march;
+        ~Restore() {
+            b->march = march;
+            free_graph(b);
+        }
+    } restore{b, march};
+    free_graph(b);
     const int cpts[] = {0, 1, 4, 10, 11};  // 0: linear tiles; + 10: the 32-register budget
     const int txs[] = {32, 64, 128, 256};
     const int tys[] = {1, 2, 4};
@@ -761,10 +919,37 @@ int lbm_batch_tune(lbm_batch* b, int32_t trial_steps, lbm_batch_config* best_out
                 }
             }
         }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    if (march) {
+        // the rows of a task, timed on single passes from the current pool into the other one, which
+        // leave the state where it is
+        b->march = true;
+        best_ms = 1e30f;
+        int best_rows = b->march_rows, r = LBM_OK;
+        for (int rows : {march_rows_for(b), 16, 24, 32, 48}) {
+            float ms = 0.0f;
+            if (r == LBM_OK) r = set_march_rows(b, rows);
+            for (int i = 0; i < 4 && r == LBM_OK; ++i) {
+                if (i == 1) cudaEventRecord(e0, b->stream);
+                r = launch_persistent(b, 3, -1, -1, b->stream, false);
+            }
+            cudaEventRecord(e1, b->stream);
+            if (r == LBM_OK) r = read_status(b);
+            if (r == LBM_OK && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess && ms / 9.0f < best_ms) {
+                best_ms = ms / 9.0f;
+                best_rows = rows;
+            }
+        }
+        if (r == LBM_OK) r = set_march_rows(b, best_rows);
+        best.ms_per_step = best_ms;
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        B_TRY(r);
+    } else {
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+    }
     B_TRY(lbm_batch_set_config(b, &best));
-    g_tune_cache[key] = best;
+    g_tune_cache[key] = {best, b->march_rows};
     if (best_out) *best_out = best;
     return LBM_OK;
 }

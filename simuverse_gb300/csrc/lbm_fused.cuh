@@ -41,19 +41,25 @@ __device__ __forceinline__ float2 from_left(float2 v, int lane) {
     return make_float2(a, lane == 0 ? a : b);
 }
 
-enum { ROW_PLAIN = 0, ROW_BOUNCE = 1, ROW_SPECIAL = 2 };
+// a row's class: 0 where every cell is plain; else the bits below, and bit FL_DIR_SHIFT + j for every
+// direction j that some cell bounces back
+enum { ROW_PLAIN = 0, ROW_MIXED = 1, ROW_FACE = 2, ROW_RARE = 4 };
 // cells whose rule needs more than a bounce-back, inlet or outflow: a moving wall beside it, or a force
 __device__ __forceinline__ bool rare_cell(unsigned f) {
     return (int)(f & FL_MAT_MASK) == LBM_EXTERNAL_FORCE || (f & FL_MOVING);
 }
-__device__ __forceinline__ bool special_cell(unsigned f) {
+__device__ __forceinline__ bool face_cell(unsigned f) {  // inlet and outflow without such a rule
     const int m = (int)(f & FL_MAT_MASK);
-    return m == LBM_INLET || m == LBM_OUTLET || rare_cell(f);
+    return (m == LBM_INLET || m == LBM_OUTLET) && !(f & FL_MOVING);
 }
 // warp-uniform class of a row whose flag words are fq (two cells per lane)
 __device__ __forceinline__ int row_class(unsigned fq) {
     if (__all_sync(0xffffffffu, (fq & (FL_PLAIN | FL_PLAIN << 16)) == (FL_PLAIN | FL_PLAIN << 16))) return ROW_PLAIN;
-    return __any_sync(0xffffffffu, special_cell(fq & 0xffffu) || special_cell(fq >> 16)) ? ROW_SPECIAL : ROW_BOUNCE;
+    // a row that is not plain: the directions that some cell bounces back come with the class
+    const int dirs = (int)(__reduce_or_sync(0xffffffffu, fq | fq >> 16) & (0x1FEu << FL_DIR_SHIFT));
+    const bool face = __any_sync(0xffffffffu, face_cell(fq & 0xffffu) || face_cell(fq >> 16));
+    const bool rare = __any_sync(0xffffffffu, rare_cell(fq & 0xffffu) || rare_cell(fq >> 16));
+    return dirs | ROW_MIXED | (face ? ROW_FACE : 0) | (rare ? ROW_RARE : 0);
 }
 __device__ __forceinline__ lbm_lattice_info fused_info(const lbm_lattice_info* info, int x, int y, int pitch, int ny) {
     const uint32_t i = (uint32_t)y * (uint32_t)pitch + (uint32_t)x;
@@ -123,22 +129,29 @@ __device__ __forceinline__ InletVel inlet_vel(unsigned fq, int xa, int xb, int y
 
 // Inlet and outflow rules on the pulled populations (bounce-back done, outflow populations in place)
 __device__ __forceinline__ void face_cells(float2 (&d)[9], unsigned fq, const InletVel& v, float omega) {
-    const BgkConst<float> ks(omega);
-#pragma unroll 1
-    for (int h = 0; h < 2; ++h) {  // one of the lane's two cells at a time: half the code
-        const unsigned f = h ? fq >> 16 : fq & 0xffffu;
-        if (special_cell(f) && !rare_cell(f)) {
+    if (__any_sync(0xffffffffu, face_cell(fq & 0xffffu))) {
+        if (face_cell(fq & 0xffffu)) {
             float e[9];
 #pragma unroll
-            for (int j = 0; j < 9; ++j) e[j] = h ? d[j].y : d[j].x;
-            if ((f & FL_MAT_MASK) == LBM_INLET) core_inlet<float>(e, h ? v.bx : v.ax, h ? v.by : v.ay);
-            else core_outlet<float>(e, ks);
+            for (int j = 0; j < 9; ++j) e[j] = d[j].x;
+            if ((fq & FL_MAT_MASK) == LBM_INLET) core_inlet<float>(e, v.ax, v.ay);
+            else core_outlet<float>(e, BgkConst<float>(omega));
 #pragma unroll
-            for (int j = 0; j < 9; ++j) {
-                if (h) d[j].y = e[j];
-                else d[j].x = e[j];
-            }
+            for (int j = 0; j < 9; ++j) d[j].x = e[j];
         }
+        __syncwarp();
+    }
+    if (__any_sync(0xffffffffu, face_cell(fq >> 16))) {
+        if (face_cell(fq >> 16)) {
+            float e[9];
+#pragma unroll
+            for (int j = 0; j < 9; ++j) e[j] = d[j].y;
+            if (((fq >> 16) & FL_MAT_MASK) == LBM_INLET) core_inlet<float>(e, v.bx, v.by);
+            else core_outlet<float>(e, BgkConst<float>(omega));
+#pragma unroll
+            for (int j = 0; j < 9; ++j) d[j].y = e[j];
+        }
+        __syncwarp();
     }
 }
 
@@ -168,6 +181,7 @@ __device__ __forceinline__ void rare_cells(const float2 (&d)[9], unsigned fq, in
 // keeps a value in registers: the compiler may not load it again where it is used
 __device__ __forceinline__ void hold(float2& v) { asm volatile("" : "+f"(v.x), "+f"(v.y)); }
 __device__ __forceinline__ void hold(int& v) { asm volatile("" : "+r"(v)); }
+__device__ __forceinline__ void hold(uint32_t& v) { asm volatile("" : "+r"(v)); }
 
 // the stored part of a row in global memory
 struct RowOut {

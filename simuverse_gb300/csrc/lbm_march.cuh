@@ -12,8 +12,9 @@
 // T = 3 moves about 26 bytes per cell and step.  The march needs no barrier, and loads are in flight
 // during two rows' arithmetic; tiles in shared memory (K = 4 steps, one copy of the region) were
 // measured slower, their load phases are exposed (4096^2 without solids: 152 against 211 GLUPS with the same arithmetic).
-// Measured, BGK, GLUPS before (one step per launch) and now: channel with disks 4096^2 91 and 163,
-// 8192^2 86 and 175; KBC 2048^2 63 and 105.  What bounds it now: 55 % of the issue slots at three warps per
+// Measured, BGK, GLUPS before (one step per launch) and now: channel with disks 4096^2 91 and 174,
+// 8192^2 86 and 186; KBC 2048^2 63 and 106.  Rows with bounce-backs cost 1.5 times a plain row, rows with an
+// inlet or outflow cell twice.  What bounds it now: 55 % of the issue slots at three warps per
 // scheduler (registers), waits for fixed latencies; DRAM at 60 to 75 % of the measured copy rate.
 //
 // Cells next to a solid bounce their own outgoing population back (a select); inlet, outflow,
@@ -44,6 +45,13 @@ __device__ __forceinline__ float2 lds_pair(uint32_t a) { return make_float2(lds_
 __device__ __forceinline__ void sts_pair(uint32_t a, float2 v) {
     asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v.x) : "memory");
     asm volatile("st.shared.f32 [%0], %1;" ::"r"(a + 128), "f"(v.y) : "memory");
+}
+// v = the word at a where m is not zero: one predicated load, no select
+__device__ __forceinline__ void lds_where(float& v, uint32_t a, unsigned m) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.shared.f32 %0, [%1];\n\t}"
+                 : "+f"(v)
+                 : "r"(a), "r"(m)
+                 : "memory");
 }
 __device__ __forceinline__ unsigned lds_u16(uint32_t a) {
     unsigned short v;
@@ -133,11 +141,11 @@ __device__ __forceinline__ void ring_pulls(MarchRing& R, int lane, int cls, unsi
     R.p4 = R.o4;
     R.p7 = from_right(R.o7, lane);
     R.p8 = from_left(R.o8, lane);
-    if (MIXED && cls == ROW_SPECIAL) {
+    if (MIXED && (cls & (ROW_FACE | ROW_RARE))) {
         if ((fq & FL_MAT_MASK) == LBM_OUTLET) d[3].x = R.o3.x;
         if (((fq >> 16) & FL_MAT_MASK) == LBM_OUTLET) d[3].y = R.o3.y;
     }
-    if (MIXED && cn == ROW_SPECIAL) {
+    if (MIXED && (cn & (ROW_FACE | ROW_RARE))) {
         if ((fn & FL_MAT_MASK) == LBM_OUTLET) R.p7.x = R.o7.x;
         if (((fn >> 16) & FL_MAT_MASK) == LBM_OUTLET) R.p7.y = R.o7.y;
     }
@@ -149,7 +157,7 @@ __device__ __forceinline__ void ring_push(MarchRing& R, const float2 (&C)[9], in
     d[2] = C[2];
     d[5] = from_left(C[5], lane);
     d[6] = from_right(C[6], lane);
-    if (MIXED && cls == ROW_SPECIAL) {
+    if (MIXED && (cls & (ROW_FACE | ROW_RARE))) {
         if ((fq & FL_MAT_MASK) == LBM_OUTLET) d[6].x = C[6].x;
         if (((fq >> 16) & FL_MAT_MASK) == LBM_OUTLET) d[6].y = C[6].y;
     }
@@ -161,6 +169,22 @@ __device__ __forceinline__ void ring_push(MarchRing& R, const float2 (&C)[9], in
     R.o8 = C[8];
 }
 
+// directions (flag bits) with e_x = 1, -1 and 0
+__host__ __device__ constexpr int dir_group(int g) {
+    return g == 0 ? (1 << 1 | 1 << 5 | 1 << 8) << FL_DIR_SHIFT
+                  : (g == 1 ? (1 << 3 | 1 << 6 | 1 << 7) << FL_DIR_SHIFT : (1 << 2 | 1 << 4) << FL_DIR_SHIFT);
+}
+// leaves what the bounce-backs of a row of class cls read in the next step: its own populations
+__device__ __forceinline__ void keep_own(uint32_t at, int cls, const float2 (&C)[9]) {
+#pragma unroll
+    for (int g = 0; g < 3; ++g) {
+        if (!(cls & dir_group(g))) continue;  // warp-uniform
+#pragma unroll
+        for (int j = 1; j < 9; ++j)
+            if (dir_group(g) >> (FL_DIR_SHIFT + INV(j)) & 1) sts_pair(at + 256 * (j - 1), C[j]);
+    }
+}
+
 // One row of one step: bounce-back (own: shared address of the cell's own outgoing population 1 of
 // the step before, `stride` bytes from one population to the next), inlet, outflow, collision, rare cells.
 template <int COLL, bool MIXED>
@@ -168,18 +192,24 @@ __device__ __forceinline__ void march_row(float2 (&d)[9], uint32_t own, int stri
                                           int y, const FusedLattice& L, const BgkConst<float2>& k, float2 (&o)[9],
                                           float2& rho, float2& nux, float2& nuy) {
     if (MIXED && cls != ROW_PLAIN) {
+        // by groups of directions, as walls ask for them: from the west, from the east, straight
 #pragma unroll
-        for (int j = 1; j < 9; ++j) {
-            const uint32_t a = own + (uint32_t)((INV(j) - 1) * stride);
-            if (fq & (1u << (FL_DIR_SHIFT + j))) d[j].x = lds_f32(a);
-            if (fq & (1u << (16 + FL_DIR_SHIFT + j))) d[j].y = lds_f32(a + 128);
+        for (int g = 0; g < 3; ++g) {
+            if (!(cls & dir_group(g))) continue;  // warp-uniform
+#pragma unroll
+            for (int j = 1; j < 9; ++j) {
+                if (!(dir_group(g) >> (FL_DIR_SHIFT + j) & 1)) continue;
+                const uint32_t a = own + (uint32_t)((INV(j) - 1) * stride);
+                lds_where(d[j].x, a, fq & (1u << (FL_DIR_SHIFT + j)));
+                lds_where(d[j].y, a + 128, fq & (1u << (16 + FL_DIR_SHIFT + j)));
+            }
         }
-        if (cls == ROW_SPECIAL) face_cells(d, fq, vel, k.omega);
+        if (cls & ROW_FACE) face_cells(d, fq, vel, k.omega);
     }
     float2 drho, jx, jy;
     core_moments<float2>(d, drho, jx, jy);
     core_collide<COLL, float2>(d, k, drho, jx, jy, o, rho, nux, nuy);
-    if (MIXED && cls == ROW_SPECIAL) rare_cells<COLL>(d, fq, xa, xb, y, L, k.omega, o, rho, nux, nuy);
+    if (MIXED && (cls & ROW_RARE)) rare_cells<COLL>(d, fq, xa, xb, y, L, k.omega, o, rho, nux, nuy);
 }
 
 // One warp: T steps of the window whose first stored column is x0 (a multiple of 4 when VEC), rows
@@ -187,7 +217,7 @@ __device__ __forceinline__ void march_row(float2 (&d)[9], uint32_t own, int stri
 template <int T, int COLL, bool VEC>
 __device__ __forceinline__ void march_window(const FusedLattice& L, const BgkConst<float2>& kin, int x0, int y0, int y1,
                                              bool macro, uint32_t smem) {
-    static_assert(T == 2 || T == 3, "fused steps");
+    static_assert(T >= 1 && T <= 3, "steps of one pass");
     constexpr int HALO = T - 1;
     constexpr int IN = 4 - HALO;  // the window's first column in a slot
     int lane = threadIdx.x & 31;
@@ -197,7 +227,8 @@ __device__ __forceinline__ void march_window(const FusedLattice& L, const BgkCon
     hold(k.one); hold(k.mone); hold(k.m15);
     const int WN = VEC ? L.pitch : L.nx;  // where columns wrap (a padded row never reaches round)
     const int xa = wrap_to(x0 - HALO + lane, WN), xb = wrap_to(x0 - HALO + 32 + lane, WN);
-    const uint32_t at = 4 * (IN + lane), kept = smem + KEPT_OFF + 4 * lane;
+    uint32_t kept = smem + KEPT_OFF + 4 * lane;
+    hold(kept);
 
     MarchLoader<VEC> ld;
     ld.init(L, x0 - 4, lane);
@@ -211,16 +242,18 @@ __device__ __forceinline__ void march_window(const FusedLattice& L, const BgkCon
 
     int yr = wrap_row(y0 - HALO, L.ny);  // wrapped row of step 1
     int ym = yr == 0 ? L.ny - 1 : yr - 1, yl = yr + 1 == L.ny ? 0 : yr + 1;
-    uint32_t sm = smem, s0 = smem + SLOT_BYTES, sp = smem + 2 * SLOT_BYTES, sn = smem + 3 * SLOT_BYTES,
-             sf = smem + 4 * SLOT_BYTES;  // rows r - 1 .. r + 3
+    // slots of rows r - 1 .. r + 3, at the lane's first cell: every access below is a constant offset away
+    uint32_t sm = smem + 4 * (IN + lane);
+    uint32_t s0 = sm + SLOT_BYTES, sp = s0 + SLOT_BYTES, sn = sp + SLOT_BYTES, sf = sn + SLOT_BYTES;
+    const uint32_t off = 4 * (IN + lane);
     int yn = yl + 1 == L.ny ? 0 : yl + 1;
-    ld.issue(L, (uint32_t)ym * (uint32_t)L.pitch, sm);
-    ld.issue(L, (uint32_t)yr * (uint32_t)L.pitch, s0);
-    ld.issue(L, (uint32_t)yl * (uint32_t)L.pitch, sp);
-    ld.issue(L, (uint32_t)yn * (uint32_t)L.pitch, sn);
+    ld.issue(L, (uint32_t)ym * (uint32_t)L.pitch, sm - off);
+    ld.issue(L, (uint32_t)yr * (uint32_t)L.pitch, s0 - off);
+    ld.issue(L, (uint32_t)yl * (uint32_t)L.pitch, sp - off);
+    ld.issue(L, (uint32_t)yn * (uint32_t)L.pitch, sn - off);
     const auto flags_of = [&](uint32_t slot, int y) {
         if constexpr (VEC) {
-            const uint32_t fa = slot + SLOT_FLAGS + 2 * (IN + lane);
+            const uint32_t fa = slot + SLOT_FLAGS - 2 * (IN + lane);
             return lds_u16(fa) | lds_u16(fa + 64) << 16;
         } else {
             const uint32_t o = (uint32_t)y * (uint32_t)L.pitch;
@@ -242,48 +275,49 @@ __device__ __forceinline__ void march_window(const FusedLattice& L, const BgkCon
         asm volatile("cp.async.wait_group 1;" ::: "memory");  // all but the row after the next one
         __syncwarp();  // the row below has arrived for every lane, and nobody reads row r - 2 any more
         const int yf = yn + 1 == L.ny ? 0 : yn + 1;
-        if (r + 2 < end) ld.issue(L, (uint32_t)yf * (uint32_t)L.pitch, sf);
+        if (r + 2 < end) ld.issue(L, (uint32_t)yf * (uint32_t)L.pitch, sf - off);
         else asm volatile("cp.async.commit_group;" ::: "memory");  // an empty group keeps the count
         f0 = fn;
         c0 = row_class(f0);
         const InletVel v0 = vn;
         fn = flags_of(sp, yl);
         vn = inlet_vel(fn, xa, xb, yl, L);
-        const int ys = T == 2 ? ym : (ym == 0 ? L.ny - 1 : ym - 1);  // row of step T
+        const int ys = T == 1 ? yr : (T == 2 ? ym : (ym == 0 ? L.ny - 1 : ym - 1));  // row of step T
 
         const auto rows = [&](auto mixed) {
             constexpr bool MIXED = decltype(mixed)::value;
             // later steps' inlet velocities are in the first-level cache by now
             const auto vel_of = [&](int cls, unsigned fq, int y) {
-                return MIXED && cls == ROW_SPECIAL ? inlet_vel(fq, xa, xb, y, L) : InletVel{0.0f, 0.0f, 0.0f, 0.0f};
+                return MIXED && (cls & ROW_FACE) ? inlet_vel(fq, xa, xb, y, L) : InletVel{0.0f, 0.0f, 0.0f, 0.0f};
             };
             float2 d1[9], d2[9], d3[9], C1[9], C2[9], o[9], rho, nux, nuy;
             // pulls from the rings first: their registers take the new rows
-            ring_pulls<MIXED>(R1, lane, c1, f1, c0, f0, d2);
-            if (T == 3) ring_pulls<MIXED>(R2, lane, c2, f2, c1, f1, d3);
+            if (T > 1) ring_pulls<MIXED>(R1, lane, c1, f1, c0, f0, d2);
+            if (T > 2) ring_pulls<MIXED>(R2, lane, c2, f2, c1, f1, d3);
 #pragma unroll
             for (int j = 0; j < 9; ++j)
-                d1[j] = lds_pair((EY(j) == 1 ? sm : (EY(j) == -1 ? sp : s0)) + at + 4 * (MARCH_RAW * j - EX(j)));
-            if (MIXED && c0 == ROW_SPECIAL) {  // outflow cells pull from their own column
-                const float2 e3 = lds_pair(s0 + at + 4 * MARCH_RAW * 3), e6 = lds_pair(sp + at + 4 * MARCH_RAW * 6),
-                             e7 = lds_pair(sm + at + 4 * MARCH_RAW * 7);
+                d1[j] = lds_pair((EY(j) == 1 ? sm : (EY(j) == -1 ? sp : s0)) + 4 * (MARCH_RAW * j - EX(j)));
+            if (MIXED && (c0 & (ROW_FACE | ROW_RARE))) {  // outflow cells pull from their own column
+                const float2 e3 = lds_pair(s0 + 4 * MARCH_RAW * 3), e6 = lds_pair(sp + 4 * MARCH_RAW * 6),
+                             e7 = lds_pair(sm + 4 * MARCH_RAW * 7);
                 if ((f0 & FL_MAT_MASK) == LBM_OUTLET) { d1[3].x = e3.x; d1[6].x = e6.x; d1[7].x = e7.x; }
                 if (((f0 >> 16) & FL_MAT_MASK) == LBM_OUTLET) { d1[3].y = e3.y; d1[6].y = e6.y; d1[7].y = e7.y; }
             }
-            march_row<COLL, MIXED>(d1, s0 + at + 4 * MARCH_RAW, 4 * MARCH_RAW, c0, f0, v0, xa, xb, yr, L, k, C1, rho, nux, nuy);
-            ring_push<MIXED>(R1, C1, lane, c1, f1, d2);
-            float2(&n2)[9] = T == 2 ? o : C2;
-            march_row<COLL, MIXED>(d2, kept, 256, c1, f1, vel_of(c1, f1, ym), xa, xb, ym, L, k, n2, rho, nux, nuy);
-            if (MIXED && c0 != ROW_PLAIN) {
-#pragma unroll
-                for (int j = 1; j < 9; ++j) sts_pair(kept + 256 * (j - 1), C1[j]);
+            march_row<COLL, MIXED>(d1, s0 + 4 * MARCH_RAW, 4 * MARCH_RAW, c0, f0, v0, xa, xb, yr, L, k,
+                                   T == 1 ? o : C1, rho, nux, nuy);
+            if constexpr (T > 1) {
+                ring_push<MIXED>(R1, C1, lane, c1, f1, d2);
+                march_row<COLL, MIXED>(d2, kept, 256, c1, f1, vel_of(c1, f1, ym), xa, xb, ym, L, k, T == 2 ? o : C2, rho,
+                                       nux, nuy);
+                if (MIXED && c0 != ROW_PLAIN) {
+                    keep_own(kept, c0, C1);
+                }
             }
-            if constexpr (T == 3) {
+            if constexpr (T > 2) {
                 ring_push<MIXED>(R2, C2, lane, c2, f2, d3);
                 march_row<COLL, MIXED>(d3, kept + 2048, 256, c2, f2, vel_of(c2, f2, ys), xa, xb, ys, L, k, o, rho, nux, nuy);
                 if (MIXED && c1 != ROW_PLAIN) {
-#pragma unroll
-                    for (int j = 1; j < 9; ++j) sts_pair(kept + 2048 + 256 * (j - 1), C2[j]);
+                    keep_own(kept + 2048, c1, C2);
                 }
             }
             if (r >= y0 + HALO) {
@@ -293,12 +327,12 @@ __device__ __forceinline__ void march_window(const FusedLattice& L, const BgkCon
                 const int xe = min(x0 + MARCH_OUT, L.nx);
                 t.sa = t.ca >= x0 && t.ca < xe;
                 t.sb = t.ca + 32 >= x0 && t.ca + 32 < xe;
-                const unsigned fs = T == 2 ? f1 : f2;
+                const unsigned fs = T == 1 ? f0 : (T == 2 ? f1 : f2);
                 store_row(L, t, !MIXED || !is_solid((int)(fs & FL_MAT_MASK)),
                           !MIXED || !is_solid((int)((fs >> 16) & FL_MAT_MASK)), macro, o, rho, nux, nuy);
             }
         };
-        if ((c0 | c1 | c2) == ROW_PLAIN) rows(std::false_type{});
+        if ((c0 | (T > 1 ? c1 : 0) | (T > 2 ? c2 : 0)) == ROW_PLAIN) rows(std::false_type{});
         else rows(std::true_type{});
 
         f2 = f1;

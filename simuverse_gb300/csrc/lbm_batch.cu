@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(32 * BM_WARPS, BM_BLOCKS)
     extern __shared__ __align__(16) unsigned char march_mem[];
     __shared__ FusedLattice lattices[BM_WARPS];
     const int wid = (int)threadIdx.x >> 5;
-    const uint32_t smem = (uint32_t)__cvta_generic_to_shared(march_mem) + (uint32_t)(wid * MARCH_SMEM);
+    const uint32_t smem = (uint32_t)__cvta_generic_to_shared(march_mem) + (uint32_t)(wid * march_smem(3));
     const int warps = (int)gridDim.x * BM_WARPS;
     for (int done = 0, pass = 0; done < nsteps; ++pass) {
         const int left = nsteps - done, T = left == 4 ? 2 : min(left, 3);
@@ -504,7 +504,7 @@ int persistent_grid(lbm_batch* b, int* grid) {
     int per_sm = 0;
     const int threads = b->march ? 32 * lbm::BM_WARPS : b->cfg.tile_threads_x * b->cfg.tile_rows;
     if (b->march) {
-        constexpr int SMEM = lbm::BM_WARPS * lbm::MARCH_SMEM;
+        constexpr int SMEM = lbm::BM_WARPS * lbm::march_smem(3);
         static lbm::PerDevice<int> fit;
         B_CK(fit.get(
             b->device,
@@ -535,7 +535,7 @@ int launch_persistent(lbm_batch* b, int nsteps, int skip_block, int skip_step, c
     std::memset(&lc, 0, sizeof(lc));
     lc.gridDim = dim3((unsigned)grid);
     lc.blockDim = b->march ? dim3(32u * lbm::BM_WARPS) : dim3((unsigned)b->cfg.tile_threads_x, (unsigned)b->cfg.tile_rows);
-    lc.dynamicSmemBytes = b->march ? lbm::BM_WARPS * lbm::MARCH_SMEM : 0;
+    lc.dynamicSmemBytes = b->march ? lbm::BM_WARPS * lbm::march_smem(3) : 0;
     lc.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;

@@ -41,12 +41,15 @@ __host__ __device__ constexpr R PW(int j) {
 //       cell c+e_k (boundary.wgsl:28-31 moved into the owning fluid cell);
 //     reference mode, solid cell: slot k is zeroed (wall-to-wall slot, see lbm_kernels.cu);
 //     physics mode, fluid cell: the pull source of direction k is solid (bounce-back).
-//   bit 13    physics mode: some bounce-back source is a moving wall
-//   bit 14    physics mode: plain fluid (bulk, ghost or code 0, no solid pull source), the
-//             cells the step kernels' warp-uniform fast path takes
+//   bit 13    physics mode: some bounce-back source is a moving wall;
+//             reference mode: fluid cell on the outer ring with a solid pull source
+//   bit 14    plain fluid, the cells the step kernels' warp-uniform fast path takes: in physics mode
+//             bulk, ghost or code 0 without a solid pull source; in reference mode fluid that
+//             neither forces, hands a population to a wall nor has bit 13
 constexpr unsigned FL_MAT_MASK = 15u;
 constexpr int FL_DIR_SHIFT = 4;
 constexpr unsigned FL_MOVING = 1u << 13;
+constexpr unsigned FL_RING = 1u << 13;
 constexpr unsigned FL_PLAIN = 1u << 14;
 __host__ __device__ constexpr unsigned plain_bit(unsigned fl) {
     return ((fl & FL_MAT_MASK) == LBM_BULK || (fl & FL_MAT_MASK) == LBM_GHOST || (fl & FL_MAT_MASK) == 0u) &&

@@ -189,34 +189,36 @@ struct RowOut {
     int ca;        // the lane's first column
     bool sa, sb;   // whether its two cells are stored
 };
+// macro field of a row's two cells; ga, gb: fluid (a solid cell's is zero)
+__device__ __forceinline__ void store_macro(const FusedLattice& L, const RowOut& t, bool ga, bool gb, float2 rho,
+                                            float2 nux, float2 nuy) {
+    const long long i = (long long)t.row + t.ca;
+    float* m = L.macro + i;
+    if (t.sa && in_bounds((unsigned long long)i, L.N, BS_FUSED_MACRO)) {
+        m[0] = ga ? rho.x : 0.0f;
+        m[(size_t)L.N] = ga ? -nux.x : 0.0f;
+        m[(size_t)2 * L.N] = ga ? -nuy.x : 0.0f;
+    }
+    if (t.sb && in_bounds((unsigned long long)(i + 32), L.N, BS_FUSED_MACRO)) {
+        m[32] = gb ? rho.y : 0.0f;
+        m[(size_t)L.N + 32] = gb ? -nux.y : 0.0f;
+        m[(size_t)2 * L.N + 32] = gb ? -nuy.y : 0.0f;
+    }
+}
 __device__ __forceinline__ void store_row(const FusedLattice& L, const RowOut& t, bool ga, bool gb, bool macro,
-                                           const float2 (&o)[9], float2 rho, float2 nux, float2 nuy) {
+                                          const float2 (&o)[9], float2 rho, float2 nux, float2 nuy) {
     // signed: the first column may lie left of the lattice where the second lies in it
     const long long i = (long long)t.row + t.ca;
-    const bool sa = t.sa && in_bounds((unsigned long long)i, L.N, BS_FUSED_STORE);
-    const bool sb = t.sb && in_bounds((unsigned long long)(i + 32), L.N, BS_FUSED_STORE);
     float* q = L.B + i;
-    if (sa && ga) {
+    if (t.sa && ga && in_bounds((unsigned long long)i, L.N, BS_FUSED_STORE)) {
 #pragma unroll
         for (int j = 0; j < 9; ++j) q[(size_t)j * L.N] = o[j].x;
     }
-    if (sb && gb) {
+    if (t.sb && gb && in_bounds((unsigned long long)(i + 32), L.N, BS_FUSED_STORE)) {
 #pragma unroll
         for (int j = 0; j < 9; ++j) q[(size_t)j * L.N + 32] = o[j].y;
     }
-    if (macro) {
-        float* m = L.macro + i;
-        if (sa) {
-            m[0] = ga ? rho.x : 0.0f;
-            m[(size_t)L.N] = ga ? -nux.x : 0.0f;
-            m[(size_t)2 * L.N] = ga ? -nuy.x : 0.0f;
-        }
-        if (sb) {
-            m[32] = gb ? rho.y : 0.0f;
-            m[(size_t)L.N + 32] = gb ? -nux.y : 0.0f;
-            m[(size_t)2 * L.N + 32] = gb ? -nuy.y : 0.0f;
-        }
-    }
+    if (macro) store_macro(L, t, ga, gb, rho, nux, nuy);
 }
 
 }  // namespace lbm

@@ -49,7 +49,17 @@ __global__ void k_build_flags(const lbm_lattice_info* __restrict__ info, uint16_
             for (int k = 1; k < 9; ++k) {
                 if (is_solid(info[(size_t)(y + EY(k)) * nx + (x + EX(k))].material)) fl |= 1u << (FL_DIR_SHIFT + k);
             }
+        } else {
+#pragma unroll
+            for (int k = 1; k < 9; ++k) {
+                const int sx = x - EX(k), sy = y - EY(k);
+                if (is_solid(info[(size_t)(sy < 0 ? ny - 1 : (sy >= ny ? 0 : sy)) * nx + (sx < 0 ? nx - 1 : (sx >= nx ? 0 : sx))].material))
+                    fl |= FL_RING;
+            }
         }
+        if (!is_solid(code) && code != LBM_INLET && code != LBM_EXTERNAL_FORCE &&
+            !(fl & (FL_RING | 0x1FFu << FL_DIR_SHIFT)))
+            fl |= FL_PLAIN;
     } else {
         if (!is_solid(code)) {
 #pragma unroll

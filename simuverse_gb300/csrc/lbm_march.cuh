@@ -67,7 +67,8 @@ constexpr int MARCH_RAW = 68;
 constexpr int SLOT_FLAGS = 9 * MARCH_RAW * 4;  // byte offset of the flag words
 constexpr int SLOT_BYTES = SLOT_FLAGS + ((MARCH_RAW * 2 + 15) / 16) * 16;
 constexpr int KEPT_OFF = 5 * SLOT_BYTES;            // own outgoing populations 1 .. 8 of steps 1 and 2
-constexpr int MARCH_SMEM = KEPT_OFF + 2 * 8 * 256;  // bytes per warp
+// bytes per warp that fuses t steps
+__host__ __device__ constexpr int march_smem(int t) { return KEPT_OFF + (t > 1 ? t - 1 : 0) * 8 * 256; }
 
 // The copies of a warp.  VEC (rows a multiple of 4 cells long): 16-byte copies of four cells, two
 // planes at a time by the two halves of the warp, then the seventeenth chunk of all nine planes;
@@ -119,6 +120,22 @@ struct MarchLoader {
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
 };
+
+// flag words of a lane's two cells in row y, whose slot address (at the lane's first cell, column `col`
+// of the slot) is `slot`
+template <bool VEC>
+__device__ __forceinline__ unsigned march_flags(const FusedLattice& L, uint32_t slot, int col, int xa, int xb, int y) {
+    if constexpr (VEC) {
+        const uint32_t fa = slot + SLOT_FLAGS - 2 * col;
+        return lds_u16(fa) | lds_u16(fa + 64) << 16;
+    } else {
+        const uint32_t o = (uint32_t)y * (uint32_t)L.pitch;
+        const bool in = in_bounds((unsigned long long)o + xa, L.N, BS_FUSED_FLAGS) &&
+                        in_bounds((unsigned long long)o + xb, L.N, BS_FUSED_FLAGS);
+        return in ? (unsigned)__ldg(L.flags + (o + (uint32_t)xa)) | (unsigned)__ldg(L.flags + (o + (uint32_t)xb)) << 16
+                  : FL_PLAIN | FL_PLAIN << 16;
+    }
+}
 
 // what a step hands to the next one between rows: outgoing populations of its last row (o0 .. o8: those
 // that the row itself or the row below pulls), and the pulls that its last row takes from above
@@ -213,7 +230,7 @@ __device__ __forceinline__ void march_row(float2 (&d)[9], uint32_t own, int stri
 }
 
 // One warp: T steps of the window whose first stored column is x0 (a multiple of 4 when VEC), rows
-// [y0, y1).  smem: the warp's MARCH_SMEM bytes (shared address, 16-byte aligned).
+// [y0, y1).  smem: the warp's march_smem(T) bytes (shared address, 16-byte aligned).
 template <int T, int COLL, bool VEC>
 __device__ __forceinline__ void march_window(const FusedLattice& L, const BgkConst<float2>& kin, int x0, int y0, int y1,
                                              bool macro, uint32_t smem) {
@@ -251,18 +268,7 @@ __device__ __forceinline__ void march_window(const FusedLattice& L, const BgkCon
     ld.issue(L, (uint32_t)yr * (uint32_t)L.pitch, s0 - off);
     ld.issue(L, (uint32_t)yl * (uint32_t)L.pitch, sp - off);
     ld.issue(L, (uint32_t)yn * (uint32_t)L.pitch, sn - off);
-    const auto flags_of = [&](uint32_t slot, int y) {
-        if constexpr (VEC) {
-            const uint32_t fa = slot + SLOT_FLAGS - 2 * (IN + lane);
-            return lds_u16(fa) | lds_u16(fa + 64) << 16;
-        } else {
-            const uint32_t o = (uint32_t)y * (uint32_t)L.pitch;
-            const bool in = in_bounds((unsigned long long)o + xa, L.N, BS_FUSED_FLAGS) &&
-                            in_bounds((unsigned long long)o + xb, L.N, BS_FUSED_FLAGS);
-            return in ? (unsigned)__ldg(L.flags + (o + (uint32_t)xa)) | (unsigned)__ldg(L.flags + (o + (uint32_t)xb)) << 16
-                      : PLAIN2;
-        }
-    };
+    const auto flags_of = [&](uint32_t slot, int y) { return march_flags<VEC>(L, slot, IN + lane, xa, xb, y); };
 
     asm volatile("cp.async.wait_group 2;" ::: "memory");  // the first two rows
     __syncwarp();

@@ -9,6 +9,9 @@
 // sum_j o_j equals the pulled density deviation exactly up to rounding.
 #pragma once
 
+#include <type_traits>
+
+#include "lbm_cell64.cuh"
 #include "lbm_common.cuh"
 #include "lbm_core.cuh"
 
@@ -286,10 +289,12 @@ __device__ __forceinline__ void bgk_plain_fast(const float (&d)[9], float omega,
 // inside a pool (the batched form) passes the pool's base pointers and its element offsets:
 // populations at pop_off, flags and info at cell_off, macro planes at 3 * cell_off; OFF is
 // their integer type (32-bit when the pool allows, which keeps the pointers out of registers).
-template <class ST, bool MACRO, int COLL = LBM_COLLISION_BGK, bool SR = false, class OFF = size_t>
+// K: the relaxation rate, or FP64 BGK's constants made from it (lbm_cell64.cuh).
+template <class ST, bool MACRO, int COLL = LBM_COLLISION_BGK, bool SR = false, class OFF = size_t,
+          class K = typename ST::R>
 __device__ __forceinline__ void phys_cell_update(const typename ST::T* __restrict__ A, typename ST::T* __restrict__ B,
                                                  uint16_t* __restrict__ flags, lbm_lattice_info* __restrict__ info,
-                                                 typename ST::R omega, int x, int y, int nx, int pitch, int ny,
+                                                 const K omega, int x, int y, int nx, int pitch, int ny,
                                                  float* __restrict__ macro, uint32_t seed = 0, OFF pop_off = 0,
                                                  OFF cell_off = 0) {
     using R = typename ST::R;
@@ -348,6 +353,11 @@ __device__ __forceinline__ void phys_cell_update(const typename ST::T* __restric
     R o[9], rho, ux, uy;
     if constexpr (core_has(COLL) && ST::dtype == LBM_DTYPE_F32)
         core_cell<R, COLL>(d, m, fl, (size_t)cc, flags, info, omega, o, rho, ux, uy);
+    else if constexpr (std::is_same<K, Bgk64>::value)
+        if (m == LBM_INLET || m == LBM_OUTLET || m == LBM_EXTERNAL_FORCE)  // few: the general collision's rules
+            phys_collide<R, COLL>(d, m, fl, (size_t)cc, flags, info, omega.omega, o, rho, ux, uy);
+        else
+            bgk64(d, omega, o, rho, ux, uy);
     else
         phys_collide<R, COLL>(d, m, fl, (size_t)cc, flags, info, omega, o, rho, ux, uy, R(ST::UNIT));
     if (MACRO && in_bounds(mc + 2 * N, end_m, BS_CELL_MACRO)) {

@@ -416,12 +416,17 @@ __global__ void __launch_bounds__(TPB, LBM_REF_MIN_BLOCKS) k_ref_step(const floa
 // ------------------------------------------------------------------------------------
 // physics-mode step (cell update in lbm_cell.cuh)
 // ------------------------------------------------------------------------------------
-// BGK and regularised fit 32 registers (full occupancy); MRT and KBC get 48
+// BGK and regularised fit 32 registers (full occupancy); MRT and KBC get 48, FP64 BGK 64
 // (SR: stochastic rounding of 16-bit stores, seed from the step counter)
-template <class ST, bool MACRO, int COLL, bool SR>
-__global__ void __launch_bounds__(TPB, (COLL == LBM_COLLISION_MRT || COLL == LBM_COLLISION_KBC) ? 10 : 16) k_phys_step(const typename ST::T* __restrict__ A, typename ST::T* __restrict__ B,
+template <int COLL, class K>
+constexpr int phys_blocks() {
+    return std::is_same<K, Bgk64>::value ? 8 : COLL == LBM_COLLISION_MRT || COLL == LBM_COLLISION_KBC ? 10 : 16;
+}
+
+template <class ST, bool MACRO, int COLL, bool SR, class K = typename ST::R>
+__global__ void __launch_bounds__(TPB, phys_blocks<COLL, K>()) k_phys_step(const typename ST::T* __restrict__ A, typename ST::T* __restrict__ B,
                                                    uint16_t* __restrict__ flags, lbm_lattice_info* __restrict__ info,
-                                                   typename ST::R omega, int nx, int ny, float* __restrict__ macro,
+                                                   const K omega, int nx, int ny, float* __restrict__ macro,
                                                    uint32_t seed) {
     const int x = blockIdx.x * TPB + threadIdx.x;
     const int y = blockIdx.y;
@@ -767,13 +772,15 @@ static cudaError_t phys_step_c(lbm_handle* h, cudaStream_t s) {
     const R omega = sizeof(R) == 8 ? (R)h->omega_d : (R)h->omega;
     // stochastic rounding exists for 16-bit storage only (validated at create)
     constexpr bool SIXTEEN = ST::dtype == LBM_DTYPE_F16 || ST::dtype == LBM_DTYPE_BF16;
+    // FP64's BGK takes its constants from the host
+    using K = std::conditional_t<ST::dtype == LBM_DTYPE_F64 && COLL == LBM_COLLISION_BGK, Bgk64, R>;
     if (SIXTEEN && h->p.rounding == LBM_ROUNDING_STOCHASTIC)
         k_phys_step<ST, MACRO, COLL, SIXTEEN><<<cell_grid(h), TPB, 0, s>>>(
             (const T*)h->buf[h->cur], (T*)h->buf[h->cur ^ 1], h->d_flags, h->d_info, omega, h->nx, h->ny, h->d_macro,
             sr_seed(h->steps, h->p.seed));
     else
-        k_phys_step<ST, MACRO, COLL, false><<<cell_grid(h), TPB, 0, s>>>(
-            (const T*)h->buf[h->cur], (T*)h->buf[h->cur ^ 1], h->d_flags, h->d_info, omega, h->nx, h->ny, h->d_macro, 0u);
+        k_phys_step<ST, MACRO, COLL, false, K><<<cell_grid(h), TPB, 0, s>>>(
+            (const T*)h->buf[h->cur], (T*)h->buf[h->cur ^ 1], h->d_flags, h->d_info, K(omega), h->nx, h->ny, h->d_macro, 0u);
     return cudaGetLastError();
 }
 

@@ -75,14 +75,14 @@ __host__ __device__ constexpr int march_smem(int t) { return KEPT_OFF + (t > 1 ?
 // else 4-byte copies of single cells.
 template <bool VEC>
 struct MarchLoader {
-    uint32_t src0, src1, src2;  // cell offsets in a row (VEC: the first two with their plane offsets)
+    uint32_t src0, src1, src2;  // cell offsets in a row (VEC: the first with its plane's, 0 or 1)
     int lane;
     // raw0: the slot's first column (a multiple of 4 when VEC), from -4 to nx
     __device__ __forceinline__ void init(const FusedLattice& L, int raw0, int ln) {
         lane = ln;
         if constexpr (VEC) {  // a chunk lies in one row: the pitch is a multiple of 4 cells, and so is raw0
             src0 = (uint32_t)(lane >> 4) * L.N + (uint32_t)wrap_to(raw0 + 4 * (lane & 15), L.pitch);
-            src1 = (uint32_t)min(lane, 8) * L.N + (uint32_t)wrap_to(raw0 + 64, L.pitch);
+            src1 = (uint32_t)wrap_to(raw0 + 64, L.pitch);
             src2 = (uint32_t)wrap_to(raw0 + 4 * min(lane, 16), L.pitch);
         } else {
             src0 = (uint32_t)wrap_to(raw0 + lane, L.nx);
@@ -98,8 +98,9 @@ struct MarchLoader {
             for (int j = 0; j < 9; j += 2)
                 if ((j < 8 || lane < 16) && in_bounds((unsigned long long)src0 + o + (unsigned long long)j * L.N + 3, 9ull * L.N, BS_FUSED_PULL))
                     cp_async_to<16>(d + 4 * MARCH_RAW * j, L.A + (size_t)j * L.N + (src0 + o));
-            if (lane < 9 && in_bounds((unsigned long long)src1 + o + 3, 9ull * L.N, BS_FUSED_PULL))
-                cp_async_to<16>(dst + 4 * MARCH_RAW * lane + 256, L.A + (src1 + o));
+            // (eight planes of 2^29 cells or more are past 32 bits)
+            if (lane < 9 && in_bounds((unsigned long long)src1 + o + 3, L.N, BS_FUSED_PULL))
+                cp_async_to<16>(dst + 4 * MARCH_RAW * lane + 256, L.A + (size_t)lane * L.N + (src1 + o));
             if (lane < 17 && in_bounds((unsigned long long)src2 + o + 3, L.N, BS_FUSED_FLAGS))
                 cp_async_to<8>(dst + SLOT_FLAGS + 8 * lane, L.flags + (src2 + o));
         } else {

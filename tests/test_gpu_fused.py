@@ -89,6 +89,27 @@ def test_counting_records_and_unlike_walls(gpu, scene, form):
         _same(a, b, n)
 
 
+def test_planes_beyond_32_bits(gpu):
+    """2^29 cells and more: eight planes are further apart than 32 bits count."""
+    import torch
+
+    from simuverse_gb300 import FluidSimulator
+
+    if torch.cuda.mem_get_info()[0] < 80 << 30:
+        pytest.skip("not enough device memory")
+    nx, ny = 32768, 16400
+    row = (0.02 * np.random.default_rng(6).standard_normal(nx + 64)).astype(np.float32)
+    u = np.stack([row[k % 61:k % 61 + nx] for k in range(ny)])
+    sums = []
+    for kernel in ("auto", "cell"):
+        s = FluidSimulator(nx, ny, mode="physics", scene="periodic", tau=0.6, kernel=kernel)
+        s.init_equilibrium(None, u, u[::-1])
+        s.step(3)
+        sums.append(s.conservation())
+        s.close()
+    assert sums[0] == sums[1]  # FP64 sums in a fixed order over the same bits
+
+
 def child_main():
     import ctypes
 

@@ -25,7 +25,7 @@ VARIANTS = {None: ("liblbm.so", "obj", []), "bounds": ("liblbm_bounds.so", "obj_
 def lib_path(variant=None) -> str:
     return os.path.join(OUT, VARIANTS[variant][0])
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-SOURCES = ["lbm_kernels.cu", "lbm_step_vec.cu", "lbm_step_bulk.cu", "lbm_step_fused.cu", "lbm_batch.cu", "lbm_noalloc.cu", "lbm_closure.cu", "lbm_view.cu", "lbm_api.cpp"]
+SOURCES = ["lbm_kernels.cu", "lbm_step_vec.cu", "lbm_step_bulk.cu", "lbm_step_fused.cu", "lbm_step_cluster.cu", "lbm_batch.cu", "lbm_noalloc.cu", "lbm_closure.cu", "lbm_view.cu", "lbm_api.cpp"]
 
 
 def _nvcc() -> str:

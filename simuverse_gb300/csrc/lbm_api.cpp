@@ -428,6 +428,8 @@ int scene_and_state_on_device(lbm_handle* h) {
     h->host_info.clear();
     h->host_info_lazy = true;
     h->no_solids = h->p.scene == LBM_SCENE_PERIODIC;
+    h->faces = h->p.scene == LBM_SCENE_CHANNEL;  // the inlet in the first column, the outflow in the last one
+    h->outlets_last = true;
     return LBM_OK;
 }
 
@@ -631,6 +633,7 @@ int lbm_create(const lbm_params* pin, lbm_handle** out) {
         r = scene_and_state_on_device(h);  // also initialises the state
     } else {
         build_scene_mask(p, h->host_info);
+        lbm::cluster_cells(h, h->host_info.data(), false);
         r = upload_info_rows(h, 0, h->ny);
         if (r == LBM_OK) r = init_state(h);
     }
@@ -685,11 +688,13 @@ int lbm_step(lbm_handle* h, int32_t nsteps) {
     if (nsteps < 0) return fail(LBM_ERR_ARG, "negative step count");
     LBM_TRY(use_device(h));
     for (int32_t s = 0; s < nsteps;) {
-        const int n = lbm::fused_steps(h, nsteps - s);
+        const int small = lbm::cluster_steps(h, nsteps - s);
+        const int n = small > 1 ? small : lbm::fused_steps(h, nsteps - s);
         const bool macro = h->p.macro_every_step || s + n == nsteps;
-        LBM_CK(n > 1 ? lbm::launch_fused(h, n, macro, h->stream) : lbm::launch_step(h, macro, h->stream));
+        if (small > 1) LBM_CK(lbm::launch_cluster(h, n, macro, h->stream));
+        else LBM_CK(n > 1 ? lbm::launch_fused(h, n, macro, h->stream) : lbm::launch_step(h, macro, h->stream));
         s += n;
-        h->cur ^= 1;
+        h->cur ^= small > 1 ? n & 1 : 1;
         h->steps += n;
         h->countdown = std::max<int64_t>(0, h->countdown - n);
         ++h->launches;
@@ -712,6 +717,7 @@ int lbm_reset(lbm_handle* h) {
     } else {
         if (h->p.mode == LBM_MODE_PHYSICS || h->p.scene == LBM_SCENE_POISEUILLE) {
             build_scene_mask(h->p, h->host_info);
+            lbm::cluster_cells(h, h->host_info.data(), false);
             h->host_info_lazy = false;
             r = upload_info_rows(h, 0, h->ny);
         }
@@ -982,6 +988,7 @@ int lbm_set_info(lbm_handle* h, const lbm_lattice_info* info) {
     h->no_solids = false;
     h->solids_agree = false;  // a new solid cell keeps what it held as fluid, another step in each buffer
     h->countdown = INT64_MAX;
+    lbm::cluster_cells(h, info, false);
     LBM_TRY(upload_info_rows(h, 0, h->ny));
     LBM_TRY(rebuild_flags(h));
     return whole_countdown(h);
@@ -1216,6 +1223,8 @@ int lbm_load(lbm_handle* h, const char* path) {
     h->host_info_lazy = false;
     h->host_mirror_valid = false;
     h->countdown = INT64_MAX;
+    lbm::cluster_cells(h, info.data(), false);
+    lbm::cluster_cells(h, hinfo.data(), true);  // its rows may be uploaded
     h->no_solids = h->solids_agree = false;
     h->cur = hd.cur & 1;
     h->tau = hd.tau;
@@ -1265,7 +1274,8 @@ int lbm_bounds_report(uint64_t* count, uint64_t* first_index, uint64_t* first_li
 #ifdef LBM_BOUNDS_CHECK
     lbm::BoundsRecord total{};
     cudaError_t (*takes[])(lbm::BoundsRecord*) = {lbm::bounds_take_kernels, lbm::bounds_take_vec,
-                                                 lbm::bounds_take_bulk, lbm::bounds_take_batch, lbm::bounds_take_fused};
+                                                 lbm::bounds_take_bulk, lbm::bounds_take_batch, lbm::bounds_take_fused,
+                                                 lbm::bounds_take_cluster};
     for (auto take : takes) {
         lbm::BoundsRecord r{};
         LBM_CK(take(&r));

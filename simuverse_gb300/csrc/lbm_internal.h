@@ -56,6 +56,9 @@ struct lbm_handle {
     // writes hold the same in both buffers
     int64_t countdown = 0;
     bool no_solids = false, solids_agree = false;
+    // and what those of small lattices ask (lbm_step_cluster.cu): no outflow cell outside the last column; any
+    // inlet or outflow cell
+    bool outlets_last = true, faces = false;
     bool stepped_since_init = false;  // macro_tex holds (0,0,0,1) right after init
     float pre_x = 0.0f, pre_y = 0.0f;  // FluidSimulator::pre_pos
     int device = 0;
@@ -117,6 +120,7 @@ cudaError_t bounds_take_vec(BoundsRecord* out);      // lbm_step_vec.cu: k_phys_
 cudaError_t bounds_take_bulk(BoundsRecord* out);     // lbm_step_bulk.cu: k_phys_step_bulk
 cudaError_t bounds_take_batch(BoundsRecord* out);    // lbm_batch.cu: the batched one-cell update
 cudaError_t bounds_take_fused(BoundsRecord* out);    // lbm_step_fused.cu: the fused steps
+cudaError_t bounds_take_cluster(BoundsRecord* out);  // lbm_step_cluster.cu: small lattices
 // one thread evaluates one index equal to its extent (no memory access): the record must show it
 cudaError_t bounds_selftest(cudaStream_t s);
 #endif
@@ -145,6 +149,11 @@ cudaError_t launch_step(lbm_handle* h, bool write_macro, cudaStream_t s);
 // fused steps (lbm_step_fused.cu): how many of the next `left` steps one launch takes (1: launch_step)
 int fused_steps(const lbm_handle* h, int left);
 cudaError_t launch_fused(lbm_handle* h, int steps, bool write_macro, cudaStream_t s);
+// the same for a small lattice (lbm_step_cluster.cu): the state ends in buffer cur ^ (steps & 1)
+int cluster_steps(const lbm_handle* h, int left);
+cudaError_t launch_cluster(lbm_handle* h, int steps, bool write_macro, cudaStream_t s);
+// h->outlets_last and h->faces of the records of a lattice small enough for it (also: and of those seen before)
+void cluster_cells(lbm_handle* h, const lbm_lattice_info* info, bool also);
 // *d_count (of h) = largest block_iter of an inlet or forcing cell's record, 0 without a positive one
 cudaError_t launch_longest_countdown(lbm_handle* h, cudaStream_t s);
 // *d_count (of h) = solid cells' slots that no step writes and that differ between the buffers

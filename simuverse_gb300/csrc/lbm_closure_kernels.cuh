@@ -49,10 +49,12 @@ __device__ __forceinline__ void ldsm_x4(unsigned (&r)[4], const unsigned* row) {
 
 // 16-byte global -> shared copy that bypasses the registers (cp.async); with full == false the
 // destination is zero-filled and nothing is read
-__device__ __forceinline__ void cp_async16(unsigned* dst, const void* src, bool full) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+__device__ __forceinline__ void cp_async16_at(unsigned dst, const void* src, bool full) {  // dst: shared address
     const int n = full ? 16 : 0;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async16(unsigned* dst, const void* src, bool full) {
+    cp_async16_at((unsigned)__cvta_generic_to_shared(dst), src, full);
 }
 __device__ __forceinline__ void cp_async_wait_all() {
     asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");

@@ -98,6 +98,11 @@ __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::be
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+__device__ __forceinline__ bool elect_one() {  // one thread of a converged warp
+    unsigned p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0u;
+}
 __device__ __forceinline__ bool bar_try(unsigned bar, unsigned parity) {
     unsigned ok;
     asm volatile(
@@ -426,64 +431,51 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
 // Weight gradients of one layer on the tensor cores (training):
 //   dW[tap][ci][co] = sum_cells x[cell + off(tap)][ci] g[cell][co],   db[co] = sum_cells g[cell][co]
 // over every cell of nimg images of H x W (W % 64 == 0; inputs outside an image read as zero),
-// as GEMMs with the cells as the K dimension: for each row tap dy, A = the three column-shifted
-// copies of the input row y + dy - 1 stacked along M (row dx * CIN + ci, a row of ones whose
-// product is db, zero rows up to 128), B = the output gradients of row y (N = COUT), D in
-// tensor memory (columns dy * COUT), accumulated over all the CTA's tiles.  A tile is 64 cells
-// of one image row (K = 64: 4 MMAs of K16 per row tap).
+// as GEMMs with the cells as the K dimension.  A tile is 64 columns of one gradient row y and of the three
+// input rows y - 1 .. y + 1 that it meets.  Per column tap dx one MMA chain multiplies A = the input
+// rows' channels stacked along M (row dy * CIN + ci, then eight rows of ones, whose product is db; what
+// follows up to 128 rows is whatever the stage holds there and is ignored), its cells starting at dx, by
+// B = the gradient row's channels (N = COUT), into the tensor-memory columns dx * COUT, accumulated over
+// all the CTA's tiles.
+// A CTA takes a contiguous range of tiles, numbered down the rows of each 64-column strip of each image.
 //
-// Sliding rows.  The tiles are numbered down the rows of each 64-column strip of each image, and
-// a CTA takes a contiguous range of them, so consecutive tiles are consecutive rows of a strip:
-// the transposed copies of an input row live in one of four slots (row r in slot (r + 1) % 4)
-// and serve the three tiles that read it.  A tile transposes one new input row (the row below),
-// or three where its strip starts, while the MMAs of the previous tile may still read theirs.
-// (A ring one tile deeper -- five slots, three gradient buffers -- measured no faster: the
-// per-tile work on the SM, not the wait for the MMAs, sets the pace.)
-//
-// Staging.  The input rows and the tile's 64 gradient cells are copied as they are stored (NHWC,
-// channels contiguous) into shared memory with cp.async, through a ring of three raw buffers (the
-// copies of the next two tiles are in flight while a tile is transposed); ldmatrix.trans turns
-// each 8-cell x 8-channel block into the canonical K-major core matrix (8 rows = channels, 16
-// bytes = 8 cells): thread t of the warp receives exactly the 4 bytes at offset 4t of the core
-// matrix, so the stores are contiguous.  Operand layout [k chunk][row][8]: the descriptor's
-// leading (K) offset is rows * 16, its stride (8-row) offset 128, as in the inference kernel.
-// Gradients are double-buffered.  Before a slot or gradient buffer is rewritten, thread 0 waits
-// (1 s limit) for the commit of the MMAs that read it: the tile two back, or the previous tile
-// where a strip starts.  Each CTA
-// writes its partial sums in the CUDA-core kernel's layout, so k_dweight_final reduces them the
+// Staging.  With channels contiguous (NHWC) a cell's channels are the M (N) direction of the operands, so
+// the MN-major canonical layout -- 8 cells x 8 channels, 16 bytes a cell -- needs no transposition:
+// cp.async writes each 16-byte chunk to its place, plane by plane of 8 channels (66 cells of 16 bytes, which
+// spreads a warp's chunks over the banks), and a column tap is an offset of 16 bytes in the
+// descriptor.  Eight warps copy into a ring of four stages; a ninth one issues the MMAs
+// and commits each tile's to the stage's "empty" barrier.  Waits are bounded (1 s).
+// Each CTA writes its partial sums in the CUDA-core kernel's layout, so k_dweight_final reduces them the
 // same way.
+//
+// What bounds it: the 16-byte copies, about one a cycle and SM (each input row is read by three tiles, from L2
+// after the first).  Transposing every tile with ldmatrix between two block barriers took 95, 84 and 79 us for
+// 8 images of 256^2 (32 x 32, 32 x 16 and 16 x 32 channels), 3300 cycles of mostly waiting a tile; this takes
+// 40, 33 and 29 us.
+// (Two gradient rows a tile, N = 2 COUT, need half the input copies, but their sums are rounded in another
+// order, which ten training steps amplify.)
 constexpr int DW_TILE = 64;
-constexpr int DW_THREADS = 256;
-constexpr int DW_TMEM_COLS = 128;
+constexpr int DW_COPIERS = 256;
+constexpr int DW_THREADS = DW_COPIERS + 32;
 
 template <int CIN, int COUT>
 struct DwLayout {
-    static constexpr int SROWS = 128;               // rows of a slot: 3 CIN shifted rows, ones, zeros
-    static constexpr int SLOT = 8 * SROWS * 16;     // [k chunk 8][128 rows][16 B]
-    static constexpr int NSLOT = 4;                 // input-row slots: 3 read + 1 being filled
-    static constexpr int NB = 2;                    // gradient buffers (and mbarriers)
-    static constexpr int XSTR = CIN * 2 + 16;       // padded: ldmatrix rows 8 cells apart hit distinct banks
-    static constexpr int GSTR = COUT * 2 + 16;
-    static constexpr int RAW_X = 3 * (DW_TILE + 2) * XSTR;
-    static constexpr int RAW = ((RAW_X + DW_TILE * GSTR + 127) / 128) * 128;
-    static constexpr int NRAW = 3;                  // raw ring depth
-    static constexpr int B_BYTES = COUT * DW_TILE * 2;
-    static constexpr int OFF_SLOT = NRAW * RAW;
-    static constexpr int OFF_B = OFF_SLOT + NSLOT * SLOT;
-    static constexpr int OFF_BAR = OFF_B + NB * B_BYTES;
-    static constexpr int OFF_TSLOT = OFF_BAR + 8 * NB;
-    static constexpr int SMEM = OFF_TSLOT + 16;
-    static_assert(3 * CIN + 1 <= SROWS, "three shifted rows and the ones row fit a slot");
-    static_assert(3 * COUT <= DW_TMEM_COLS, "accumulators fit the allocation");
-    static_assert(OFF_SLOT % 128 == 0 && OFF_B % 128 == 0 && OFF_BAR % 8 == 0, "alignment");
+    static constexpr int XC = CIN / 8, GC = COUT / 8;   // 8-channel groups
+    static constexpr int COLS = DW_TILE + 2;
+    static constexpr int PLANE_B = COLS * 16;           // [cell][16 B] of one group of one row
+    static constexpr int OFF_ONES = 3 * XC * PLANE_B;   // a plane of ones, after the input's [row][group]
+    static constexpr int OFF_G = OFF_ONES + PLANE_B;    // gradient planes
+    static constexpr int STAGE = (3 * XC + 1 + GC > 16 ? 3 * XC + 1 + GC : 16) * PLANE_B;  // (M = 128 reads sixteen)
+        static constexpr int NSTAGE = 4;                    // (six or eight measured 1 to 4 % slower)
+    static constexpr int OFF_BAR = NSTAGE * STAGE;      // full[NSTAGE], empty[NSTAGE], done
+    static constexpr int OFF_TSLOT = OFF_BAR + 8 * (2 * NSTAGE + 1);
+    static constexpr int SMEM = OFF_TSLOT + 8;
+    static constexpr int TMEM = 4 * COUT;               // three column taps are used; it comes in powers of two
+    static_assert(3 * CIN + 8 <= 128, "three input rows and the ones fit M");
+    static_assert(STAGE % 16 == 0 && OFF_BAR % 8 == 0, "alignment");
+    static_assert(TMEM == 64 || TMEM == 128, "tensor memory comes in powers of two");
     static_assert(SMEM <= 227 * 1024, "one CTA per SM");
 };
-
-__device__ __forceinline__ void ldsm_x4_trans(unsigned (&r)[4], unsigned addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
-}
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(DW_THREADS, 1)
@@ -491,215 +483,146 @@ __global__ void __launch_bounds__(DW_THREADS, 1)
                  float* __restrict__ partials, int* __restrict__ status) {
     using L = DwLayout<CIN, COUT>;
     extern __shared__ __align__(128) unsigned char sm[];
-    __shared__ int s_ok;
+    __shared__ int s_fail, s_ok;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const unsigned bar0 = su32(sm + L::OFF_BAR);  // one mbarrier per gradient buffer, 8 bytes apart
+    const unsigned full0 = su32(sm + L::OFF_BAR), empty0 = full0 + 8 * L::NSTAGE, done = empty0 + 8 * L::NSTAGE;
     unsigned* tslot = reinterpret_cast<unsigned*>(sm + L::OFF_TSLOT);
     const int tiles_x = W / DW_TILE, ntiles = nimg * tiles_x * H;
-    // this CTA's tiles: a contiguous range of t = (img * tiles_x + strip) * H + y
+    // this CTA's tiles: a contiguous range of t = (img * tiles_x + strip) * H + y, one at least
     const int G = (int)gridDim.x;
     const int t_begin = (int)(((long long)ntiles * blockIdx.x) / G), t_end = (int)(((long long)ntiles * (blockIdx.x + 1)) / G);
+    const int count = t_end - t_begin;
 
-    // rows of the slots that no tile writes: the ones row (db) and the zero rows
-    for (int i = tid; i < L::NSLOT * 8 * (L::SROWS - 3 * CIN); i += DW_THREADS) {
-        const int per = 8 * (L::SROWS - 3 * CIN);
-        const int sl = i / per, rem = i % per, kc = rem / (L::SROWS - 3 * CIN), m = 3 * CIN + rem % (L::SROWS - 3 * CIN);
-        const unsigned v = m == 3 * CIN ? 0x3F803F80u : 0u;  // BF16 1.0 pairs
-        *reinterpret_cast<uint4*>(sm + L::OFF_SLOT + sl * L::SLOT + (kc * L::SROWS + m) * 16) = make_uint4(v, v, v, v);
-    }
+    for (int i = tid; i < L::NSTAGE * L::COLS; i += DW_THREADS)  // BF16 1.0
+        *reinterpret_cast<uint4*>(sm + i / L::COLS * L::STAGE + L::OFF_ONES + i % L::COLS * 16) =
+            make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
     if (tid == 0) {
-        for (int k = 0; k < L::NB; ++k) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8 * k) : "memory");
+        s_fail = 0;
+        for (int k = 0; k < L::NSTAGE; ++k) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full0 + 8 * k), "r"(DW_COPIERS) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty0 + 8 * k) : "memory");
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(done) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(tslot)),
-                     "r"(DW_TMEM_COLS)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(tslot)), "r"(L::TMEM)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-
-    // raw copies of tile t into raw buffer b: the input rows it needs first (rows y - 1 .. y + 1
-    // into raw rows 0 .. 2 where its strip starts in this CTA, else row y + 1 into raw row 2) and
-    // its 64 gradient cells.  Thread tid copies the 16-byte chunks tid, tid + 256, ... of the
-    // buffer, the same in every tile.
-    constexpr int XC = CIN / 8, GC = COUT / 8;
-    constexpr int NXCH = 3 * (DW_TILE + 2) * XC, NGCH = DW_TILE * GC;
-    constexpr int NCOPY = (NXCH + NGCH + DW_THREADS - 1) / DW_THREADS;
-    int crow[NCOPY], ccol[NCOPY];  // input chunk: raw row, column (-1: a gradient chunk; -2: none)
-    unsigned coff[NCOPY], soff[NCOPY];  // channel offset within the cell / smem byte offset
-#pragma unroll
-    for (int k = 0; k < NCOPY; ++k) {
-        const int q = tid + k * DW_THREADS;
-        if (q < NXCH) {
-            const int cc = q % XC, col = (q / XC) % (DW_TILE + 2), r = q / (XC * (DW_TILE + 2));
-            crow[k] = r;
-            ccol[k] = col;
-            coff[k] = (unsigned)(cc * 8);
-            soff[k] = (unsigned)((r * (DW_TILE + 2) + col) * L::XSTR + cc * 16);
-        } else if (q < NXCH + NGCH) {
-            const int qq = q - NXCH, cc = qq % GC, cell = qq / GC;
-            crow[k] = -1;
-            ccol[k] = cell;
-            coff[k] = (unsigned)(cc * 8);
-            soff[k] = (unsigned)(L::RAW_X + cell * L::GSTR + cc * 16);
-        } else {
-            crow[k] = -2;
-            ccol[k] = 0;
-            coff[k] = 0;
-            soff[k] = 0;
-        }
-    }
-    auto starts = [&](int t) { return t == t_begin || t % H == 0; };  // a strip starts: three new rows
-    auto stage = [&](int t, int b) {
-        const int y = t % H, strip = t / H, img = strip / tiles_x, x0 = (strip % tiles_x) * DW_TILE;
-        const int first = starts(t) ? 0 : 2;
-        unsigned char* raw = sm + b * L::RAW;
-        const size_t rowx = ((size_t)img * H + y) * W;  // cell index of (img, y, 0)
-#pragma unroll
-        for (int k = 0; k < NCOPY; ++k) {
-            if (crow[k] >= first) {
-                const int gy = y + crow[k] - 1, gx = x0 + ccol[k] - 1;
-                const bool in = gy >= 0 && gy < H && gx >= 0 && gx < W;
-                const __nv_bfloat16* src =
-                    in ? x + (size_t)((long long)rowx + (long long)(crow[k] - 1) * W + gx) * CIN + coff[k] : x;
-                cp_async16(reinterpret_cast<unsigned*>(raw + soff[k]), src, in);
-            } else if (crow[k] == -1) {
-                cp_async16(reinterpret_cast<unsigned*>(raw + soff[k]), g + (rowx + x0 + ccol[k]) * COUT + coff[k], true);
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    // operands of tile t from raw buffer rb: each new input row r (raw row r - y + 1) into slot
-    // (r + 1) % 4 as three column-shifted copies (slot row dx * CIN + ci holds the cells shifted
-    // by dx - 1), and the gradients into gradient buffer gb.  One ldmatrix.x4.trans covers 4
-    // consecutive k chunks of one 8-row group; the lane's part of the source address is a
-    // constant, the rest is warp-uniform.
-    constexpr int OPR = 3 * XC * 2, OPB = GC * 2;  // ops per input row, per gradient row
-    const unsigned lane_src_x = (unsigned)(((lane >> 3) * 8 + (lane & 7)) * L::XSTR);
-    const unsigned lane_src_g = (unsigned)(((lane >> 3) * 8 + (lane & 7)) * L::GSTR);
-    auto transpose = [&](int t, int rb, int gb) {
-        const int y = t % H;
-        const int first = starts(t) ? 0 : 2, nops = (3 - first) * OPR + OPB;
-        const unsigned rx = su32(sm + rb * L::RAW);
-        unsigned char* S = sm + L::OFF_SLOT + 4 * lane;
-        unsigned char* Bm = sm + L::OFF_B + gb * L::B_BYTES + 4 * lane;
-        for (int op = warp; op < nops; op += DW_THREADS / 32) {
-            unsigned r[4];
-            unsigned char* dst;
-            unsigned stride;
-            if (op < (3 - first) * OPR) {
-                const int rr = first + op / OPR, o = op % OPR;  // raw row, op within the row
-                const int kh = o & 1, cg = (o >> 1) % XC, dx = (o >> 1) / XC;
-                ldsm_x4_trans(r, rx + lane_src_x + (unsigned)((rr * (DW_TILE + 2) + kh * 32 + dx) * L::XSTR + cg * 16));
-                const int slot = (y + rr) % L::NSLOT;  // input row y + rr - 1
-                dst = S + slot * L::SLOT + ((kh * 4) * L::SROWS + dx * CIN + cg * 8) * 16;
-                stride = L::SROWS * 16;
-            } else {
-                const int q = op - (3 - first) * OPR, kh = q & 1, ng = q >> 1;
-                ldsm_x4_trans(r, rx + L::RAW_X + lane_src_g + (unsigned)((kh * 32) * L::GSTR + ng * 16));
-                dst = Bm + ((kh * 4) * COUT + ng * 8) * 16;
-                stride = COUT * 16;
-            }
-#pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4) *reinterpret_cast<unsigned*>(dst + q4 * stride) = r[q4];
-        }
-    };
-
     fence_async_smem();
     fence_before();
     __syncthreads();
     fence_after();
     const unsigned tmem = *tslot;
-    constexpr uint32_t ID = idesc_bf16(128, COUT);
-    // operand descriptors of slot 0 and gradient buffer 0 at k chunk 0 (shared memory is below
-    // 256 KB, so adding an offset / 16 to the start address field never carries out of it)
-    const uint64_t a_desc0 = sdesc(su32(sm + L::OFF_SLOT), L::SROWS * 16, 128);
-    const uint64_t b_desc0 = sdesc(su32(sm + L::OFF_B), COUT * 16, 128);
-    bool alive = true;
-    int i = 0, last = -1;
-    // the copies of the first two tiles (an empty group when there is no second tile, so that
-    // one group per tile is always outstanding)
-    if (t_begin < t_end) stage(t_begin, 0);
-    if (t_begin + 1 < t_end) stage(t_begin + 1, 1);
-    else asm volatile("cp.async.commit_group;" ::: "memory");
-    for (int t = t_begin; t < t_end; ++t, ++i) {
-        const int b = i % L::NB;
-        asm volatile("cp.async.wait_group 1;" ::: "memory");  // tile i's copies (tile i + 1's may run)
-        if (tid == 0) {
-            // the slot this tile fills and gradient buffer b were last read by tile i - NB; where a
-            // strip starts, three slots are refilled: wait for the previous tile (and so all)
-            bool ok = i < L::NB || bar_wait_bounded(bar0 + 8 * b, ((i - L::NB) / L::NB) & 1);
-            if (ok && starts(t) && i >= 1) ok = bar_wait_bounded(bar0 + 8 * ((i - 1) % L::NB), ((i - 1) / L::NB) & 1);
-            s_ok = ok ? 1 : 0;
-        }
-        __syncthreads();
-        if (!s_ok) {
-            alive = false;
-            break;
-        }
-        transpose(t, i % L::NRAW, b);
-        // raw buffer (i + 2) % 3 was last read by the transposes of tile i - 1
-        if (t + 2 < t_end) stage(t + 2, (i + 2) % L::NRAW);
-        else asm volatile("cp.async.commit_group;" ::: "memory");
-        fence_async_smem();
-        fence_before();
-        __syncthreads();
-        if (tid == 0) {
-            fence_after();
-            const int y = t % H;
-            // descriptors differ only in their start address field (address / 16, low bits)
+
+    if (warp < DW_COPIERS / 32) {
+        // A thread copies the same chunks of every tile: their offsets from the tile's first cell, and to
+        // the stage, with the image borders that put a chunk outside in the low bits.
+        constexpr int NX = 3 * L::COLS * L::XC, NG = DW_TILE * L::GC, KX = (NX + DW_COPIERS - 1) / DW_COPIERS;
+        static_assert(NG <= DW_COPIERS && NX > (KX - 1) * DW_COPIERS, "one gradient chunk a thread");
+        enum { LEFT = 1, RIGHT = 2, ABOVE = 4, BELOW = 8 };
+        int from[KX];
+        unsigned to[KX];
 #pragma unroll
-            for (int dy = 0; dy < 3; ++dy) {
-                const uint64_t ad0 = a_desc0 + (uint64_t)((((y + dy) % L::NSLOT) * L::SLOT) >> 4);  // input row y + dy - 1
+        for (int k = 0; k < KX; ++k) {
+            const int q = tid + k * DW_COPIERS, cg = q % L::XC, cell = q / L::XC % L::COLS, r = q / (L::XC * L::COLS);
+            from[k] = ((r - 1) * W + cell - 1) * CIN + cg * 8;
+            to[k] = (unsigned)((r * L::XC + cg) * L::PLANE_B + cell * 16) | (cell == 0 ? LEFT : 0) |
+                    (cell == L::COLS - 1 ? RIGHT : 0) | (r == 0 ? ABOVE : 0) | (r == 2 ? BELOW : 0);
+        }
+        const int gcell = tid / L::GC, gcg = tid % L::GC;
+        const unsigned sm0 = su32(sm), gto = (unsigned)(L::OFF_G + gcg * L::PLANE_B + gcell * 16);
+        int y = t_begin % H, x0 = t_begin / H % tiles_x * DW_TILE;
+        size_t row0 = (size_t)(t_begin / H / tiles_x) * H * W;  // the image's first cell
+        for (int i = 0; i < count; ++i) {
+            const int b = i % L::NSTAGE;
+            if (i >= L::NSTAGE && !__all_sync(0xffffffffu, bar_wait_bounded(empty0 + 8 * b, (i / L::NSTAGE - 1) & 1))) {
+                s_fail = 1;
+                break;
+            }
+            const size_t cell0 = row0 + (size_t)y * W + x0;
+            const __nv_bfloat16 *xt = x + cell0 * CIN, *gt = g + (cell0 + gcell) * COUT + gcg * 8;
+            const unsigned border = (x0 == 0 ? LEFT : 0u) | (x0 + DW_TILE == W ? RIGHT : 0u) | (y == 0 ? ABOVE : 0u) | (y == H - 1 ? BELOW : 0u);
+            const unsigned stage = sm0 + b * L::STAGE;
+#pragma unroll
+            for (int k = 0; k < KX; ++k) {
+                if (k == KX - 1 && tid + k * DW_COPIERS >= NX) break;
+                const bool in = !(to[k] & border);
+                cp_async16_at(stage + (to[k] & ~15u), in ? xt + from[k] : x, in);
+            }
+            if (NG == DW_COPIERS || tid < NG) cp_async16_at(stage + gto, gt, true);
+            if (++y == H) {
+                y = 0;
+                if ((x0 += DW_TILE) == W) {
+                    x0 = 0;
+                    row0 += (size_t)H * W;
+                }
+            }
+            // arrives when this thread's copies so far are in shared memory
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full0 + 8 * b) : "memory");
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+        constexpr uint32_t ID = idesc_bf16(128, COUT) | 1u << 15 | 1u << 16;  // both operands MN-major
+        // MN-major: the leading offset is from 8 cells to the next, the stride from 8 channels to the next
+        const uint64_t a0 = sdesc(su32(sm), 128, L::PLANE_B), b0 = sdesc(su32(sm + L::OFF_G), 128, L::PLANE_B);
+        // the warp walks the tiles together, so that descriptors are warp-uniform values, and one
+        // elected thread issues (issuing from a lane of a divergent warp was the bottleneck)
+        int b = 0;
+        unsigned phase = 0u;
+        for (int i = 0; i < count; ++i) {
+            if (!__all_sync(0xffffffffu, bar_wait_bounded(full0 + 8 * b, phase))) {
+                s_fail = 1;
+                break;
+            }
+            fence_async_smem();  // the copies went through the generic proxy (a fence by the copiers would drain their queue)
+            fence_after();
+            const uint64_t as = a0 + (uint64_t)(b * (L::STAGE >> 4)), bs = b0 + (uint64_t)(b * (L::STAGE >> 4));
+            if (elect_one()) {
 #pragma unroll
                 for (int ks = 0; ks < DW_TILE / 16; ++ks)
-                    mma(tmem + (unsigned)(dy * COUT), ad0 + (uint64_t)((2 * ks * L::SROWS * 16) >> 4),
-                        b_desc0 + (uint64_t)((b * L::B_BYTES + 2 * ks * COUT * 16) >> 4), ID, (i > 0 || ks > 0) ? 1u : 0u);
-            }
-            commit(bar0 + 8 * b);
-        }
-        last = i;
-    }
-    // the last commit covers every MMA of the CTA
-    if (tid == 0) s_ok = (last < 0 || bar_wait_bounded(bar0 + 8 * (last % L::NB), (last / L::NB) & 1)) ? 1 : 0;
-    __syncthreads();
-    if (!s_ok) alive = false;
-    if (alive && last >= 0) {
-        fence_after();
-        // accumulator rows: row tap dy's tile, row dx * CIN + ci = tap (3 dy + dx), channel ci;
-        // row 3 CIN of every tile is db (read from dy = 1)
-        const int lane_q = warp & 3, half = warp >> 2;
-        float* p = partials + (size_t)blockIdx.x * (9 * CIN * COUT + COUT);
-        for (int dy = half; dy < 3; dy += 2) {
-            const int m = lane_q * 32 + lane;
 #pragma unroll
-            for (int c0 = 0; c0 < COUT; c0 += 16) {
+                    for (int dx = 0; dx < 3; ++dx)
+                        mma(tmem + (unsigned)(dx * COUT), as + (uint64_t)(16 * ks + dx), bs + (uint64_t)(16 * ks), ID, i > 0 || ks > 0);
+                commit(empty0 + 8 * b);
+            }
+            __syncwarp();
+            if (++b == L::NSTAGE) {
+                b = 0;
+                phase ^= 1u;
+            }
+        }
+        if (elect_one()) commit(done);  // covers every MMA of the CTA
+        __syncwarp();
+    }
+    __syncthreads();
+    if (tid == 0) s_ok = bar_wait_bounded(done, 0) && !s_fail;
+    __syncthreads();
+    if (s_ok) {
+        fence_after();
+        if (warp < 8) {
+            const int quarter = warp & 3, m = quarter * 32 + lane, dy = m / CIN, ci = m % CIN;
+            float* p = partials + (size_t)blockIdx.x * (9 * CIN * COUT + COUT);
+            for (int q = warp >> 2; q < 3 * COUT / 16; q += 2) {
                 float v[16];
-                tmem_ld16(tmem + ((unsigned)(lane_q * 32) << 16) + (unsigned)(dy * COUT + c0), v);
-                float* o = m < 3 * CIN ? p + (size_t)(dy * 3 * CIN + m) * COUT + c0
-                                       : (m == 3 * CIN && dy == 1 ? p + 9 * CIN * COUT + c0 : nullptr);
+                tmem_ld16(tmem + ((unsigned)(quarter * 32) << 16) + (unsigned)(16 * q), v);
+                const int dx = 16 * q / COUT, co = 16 * q % COUT;
+                float* o = dy < 3 ? p + (size_t)((dy * 3 + dx) * CIN + ci) * COUT + co
+                                  : (m == 3 * CIN && dx == 1 ? p + 9 * CIN * COUT + co : nullptr);
                 if (o != nullptr)
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) o[j] = v[j];
+                    for (int k = 0; k < 16; k += 4) *reinterpret_cast<float4*>(o + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
             }
         }
-    } else if (last < 0) {  // no tile: zero partials
-        float* p = partials + (size_t)blockIdx.x * (9 * CIN * COUT + COUT);
-        for (int k = tid; k < 9 * CIN * COUT + COUT; k += DW_THREADS) p[k] = 0.0f;
+    } else if (tid == 0) {
+        atomicExch(status, LBM_ERR_TIMEOUT);  // (the MMAs in flight had their second above)
     }
-    if (!alive) {  // a wait ran out: record it and let the MMAs in flight finish before freeing
-        if (tid == 0) {
-            atomicExch(status, LBM_ERR_TIMEOUT);
-            if (last >= 0) bar_wait_bounded(bar0 + 8 * (last % L::NB), (last / L::NB) & 1);
-        }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
     fence_before();
     __syncthreads();
     if (warp == 0) {
         fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(DW_TMEM_COLS)
-                     : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(L::TMEM) : "memory");
     }
 }
 

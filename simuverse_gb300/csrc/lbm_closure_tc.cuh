@@ -139,6 +139,26 @@ __device__ __forceinline__ void tmem_ld16(unsigned taddr, float (&v)[16]) {
     for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
 }
 
+// two such rows with one wait
+__device__ __forceinline__ void tmem_ld16x2(unsigned ta, unsigned tb, float (&a)[16], float (&b)[16]) {
+    unsigned r[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]),
+          "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]),
+          "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(ta), "r"(tb)
+        : "memory");
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        a[j] = __uint_as_float(r[j]);
+        b[j] = __uint_as_float(r[16 + j]);
+    }
+}
+
 // zeros into 16 / 8 consecutive accumulator columns of this thread's lane
 __device__ __forceinline__ void tmem_zero16(unsigned taddr) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(
@@ -275,43 +295,39 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
     unsigned parity = 0u;
     bool alive = true;
 
-    // the populations of input row a (lattice row ys - 3 + a, wrapped) at this thread's positions
-    // tid and tid + TC_THREADS (< POS), loaded ahead of their use
-    constexpr int NP = (POS + TC_THREADS - 1) / TC_THREADS;
-    float pre[NP][9];
+    // the populations of input row a (lattice row ys - 3 + a, wrapped) at this thread's position
+    // (< POS), loaded ahead of their use: the second warpgroup has the first 128 positions, as the first
+    // one writes the projected outputs (with both on the first, and a wait for each layer's accumulators, a
+    // call on 1024^2 took 89.7 us; now 88.2.  What bounds it: a step's MMAs and its epilogues take turns,
+    // the tensor pipe is busy for 41 % with two blocks on the SM)
+    static_assert(POS <= TC_THREADS, "one position a thread");
+    const int fp = (tid + TC_THREADS / 2) % TC_THREADS;
+    float pre[9];
     auto load_row = [&](int a) {
         const int gy = ((ys - 3 + a) % ny + ny) % ny;
-#pragma unroll
-        for (int k = 0; k < NP; ++k) {
-            const int p = tid + k * TC_THREADS;
-            if (p < POS) load_dev(d, N, (size_t)gy * nx + ((x0 - 3 + p) % nx + nx) % nx, pre[k]);
-        }
+        if (fp < POS) load_dev(d, N, (size_t)gy * nx + ((x0 - 3 + fp) % nx + nx) % nx, pre);
     };
     // features of the prefetched row into input buffer a % 2
     auto store_features = [&](int a) {
+        if (fp >= POS) return;
         unsigned char* row = ring_in + (a % 2) * IN_ROW;
+        float v[9];
 #pragma unroll
-        for (int k = 0; k < NP; ++k) {
-            const int p = tid + k * TC_THREADS;
-            if (p >= POS) continue;
-            float v[9];
+        for (int i = 0; i < 9; ++i) v[i] = pre[i];
+        if (inputs == LBM_CLOSURE_INPUT_EQ) {
+            float n[9];
 #pragma unroll
-            for (int i = 0; i < 9; ++i) v[i] = pre[k][i];
-            if (inputs == LBM_CLOSURE_INPUT_EQ) {
-                float n[9];
+            for (int i = 0; i < 9; ++i) n[i] = v[i];
+            non_equilibrium(n);
 #pragma unroll
-                for (int i = 0; i < 9; ++i) n[i] = v[i];
-                non_equilibrium(n);
-#pragma unroll
-                for (int i = 0; i < 9; ++i) v[i] -= n[i];
-            } else {
-                non_equilibrium(v);
-            }
-            *reinterpret_cast<uint4*>(row + p * 16) =
-                make_uint4(pack_bf16x2(s_in * v[0], s_in * v[1]), pack_bf16x2(s_in * v[2], s_in * v[3]),
-                           pack_bf16x2(s_in * v[4], s_in * v[5]), pack_bf16x2(s_in * v[6], s_in * v[7]));
-            *reinterpret_cast<uint4*>(row + PLANE + p * 16) = make_uint4(pack_bf16x2(s_in * v[8], 0.0f), 0u, 0u, 0u);
+            for (int i = 0; i < 9; ++i) v[i] -= n[i];
+        } else {
+            non_equilibrium(v);
         }
+        *reinterpret_cast<uint4*>(row + fp * 16) =
+            make_uint4(pack_bf16x2(s_in * v[0], s_in * v[1]), pack_bf16x2(s_in * v[2], s_in * v[3]),
+                       pack_bf16x2(s_in * v[4], s_in * v[5]), pack_bf16x2(s_in * v[6], s_in * v[7]));
+        *reinterpret_cast<uint4*>(row + PLANE + fp * 16) = make_uint4(pack_bf16x2(s_in * v[8], 0.0f), 0u, 0u, 0u);
     };
     const auto slot = [](int row) { return ((row % 3) + 3) % 3; };
 
@@ -349,23 +365,20 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
         bar_try(bar, parity);  // complete: acquire the phase in every thread
         parity ^= 1u;
         fence_after();
-        if (m1) {  // layer-1 row a - 1 complete (rows 1 .. TC_ROWS + 4 are used)
-            const unsigned t = tmem + lane_off + TM_L1 + 32 * slot(a - 1) + 16 * half;
-            if (a - 1 >= 1) {
-                float v[16];
-                tmem_ld16(t, v);
-                store_hidden16(ring_l1 + ((a - 1) % 2) * H_ROW, mrow + 1, half, v, bias);
+        if (m1 || m2) {
+            // layer-1 row a - 1 (rows 1 .. TC_ROWS + 4 are used) and layer-2 row a - 3 (2 .. TC_ROWS + 3) are complete
+            const unsigned t1 = tmem + lane_off + TM_L1 + 32 * slot(a - 1) + 16 * half;
+            const unsigned t2 = tmem + lane_off + TM_L2 + 32 * slot(a - 3) + 16 * half;
+            float v1[16], v2[16];
+            tmem_ld16x2(t1, t2, v1, v2);
+            if (m1) {
+                if (a - 1 >= 1) store_hidden16(ring_l1 + ((a - 1) % 2) * H_ROW, mrow + 1, half, v1, bias);
+                tmem_zero16(t1);
             }
-            tmem_zero16(t);
-        }
-        if (m2) {  // layer-2 row a - 3 complete (rows 2 .. TC_ROWS + 3 are used)
-            const unsigned t = tmem + lane_off + TM_L2 + 32 * slot(a - 3) + 16 * half;
-            if (a - 3 >= 2) {
-                float v[16];
-                tmem_ld16(t, v);
-                store_hidden16(ring_l2 + ((a - 3) % 2) * H_ROW, mrow + 1, half, v, bias + 32);
+            if (m2) {
+                if (a - 3 >= 2) store_hidden16(ring_l2 + ((a - 3) % 2) * H_ROW, mrow + 1, half, v2, bias + 32);
+                tmem_zero16(t2);
             }
-            tmem_zero16(t);
         }
         if (m3) {  // layer-3 row a - 5 complete: output row ys + a - 8 (rows 3 .. TC_ROWS + 2)
             const int p = mrow + 1, oy = ys + a - 8, ox = x0 - 3 + p;
@@ -640,9 +653,12 @@ __global__ void __launch_bounds__(DW_THREADS, 1)
 // row taps' weights side by side (N = 3 COUT), the row-tap blocks stored in the order [2, 1, 0, 2,
 // 1] so that output row o always lands in accumulator slot o mod 3.  After input row r the output
 // row r - 1 is complete: its slot is read, the epilogue written to global memory and the slot
-// zeroed.  Input rows are double-buffered and copied with cp.async while the MMAs of the row
-// before run; thread 0 waits (1 s limit) for each row's commit, and a wait that runs out records
-// LBM_ERR_TIMEOUT, waits (bounded) for the MMAs in flight and frees the tensor memory.
+// zeroed.  Input rows are copied two ahead with cp.async, by warps 1 to 7: thread 0 fences them to
+// the async proxy when they have landed and issues the MMAs, as a fence would drain a copier's queue.  The mask
+// of the output row is loaded while the MMAs run.  Thread 0 waits (1 s limit) for each row's commit, and a
+// wait that runs out records LBM_ERR_TIMEOUT, waits (bounded) for the MMAs in flight and frees the
+// tensor memory.  (The five calls of a training step on 8 x 256^2 took 148 us with every thread copying and
+// fencing one row ahead, now 145; the turns of MMAs and epilogue bound them.)
 constexpr int CONV_TC_ROWS = 8;
 constexpr int CONV_TC_THREADS = 256;
 constexpr int CONV_TC_TMEM = 128;
@@ -651,7 +667,8 @@ template <int CIN, int COUT>
 struct ConvTcLayout {
     static constexpr int GIN = CIN / 8;                       // 8-channel groups of an input row
     static constexpr int IN_ROW = GIN * PLANE;                // [group][130 positions][16 B]
-    static constexpr int OFF_W = 2 * IN_ROW;                  // [dx 3][group][block 5][cout][16 B]
+    static constexpr int NROW = 3;                            // input rows: one read, two on their way
+    static constexpr int OFF_W = NROW * IN_ROW;               // [dx 3][group][block 5][cout][16 B]
     static constexpr int W_BYTES = 3 * GIN * 5 * COUT * 16;
     static constexpr int OFF_BIAS = OFF_W + W_BYTES;
     static constexpr int OFF_BAR = OFF_BIAS + COUT * 4;
@@ -700,7 +717,7 @@ __global__ void __launch_bounds__(CONV_TC_THREADS, 4)
     // input row gy (zero outside the image) into ring buffer b: group g, position p = column x0 - 1 + p
     auto stage = [&](int gy, int b) {
         unsigned char* row = ring + b * L::IN_ROW;
-        for (int i = tid; i < L::GIN * POS; i += CONV_TC_THREADS) {
+        for (int i = tid - 32; i < L::GIN * POS && warp > 0; i += CONV_TC_THREADS - 32) {
             const int p = i % POS, g = i / POS, gx = x0 - 1 + p;
             const bool ok = gy >= 0 && gy < H && gx >= 0 && gx < W;
             const __nv_bfloat16* src = ok ? in + (img_off + (size_t)gy * W + gx) * CIN + g * 8 : in;
@@ -709,6 +726,7 @@ __global__ void __launch_bounds__(CONV_TC_THREADS, 4)
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     stage(y0 - 1, 0);
+    stage(y0, 1);
     fence_before();
     __syncthreads();
     fence_after();
@@ -723,8 +741,8 @@ __global__ void __launch_bounds__(CONV_TC_THREADS, 4)
         else tmem_zero8(tmem + lane_off + k * COUT + half * HC);
     }
     tmem_wait_st();
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    fence_async_smem();
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    fence_async_smem();  // the weights
     fence_before();
     __syncthreads();
     unsigned parity = 0u;
@@ -733,11 +751,22 @@ __global__ void __launch_bounds__(CONV_TC_THREADS, 4)
     for (int a = 0; a < nrows + 2; ++a) {  // input row y0 - 1 + a
         const int gy = y0 - 1 + a;
         if (tid == 0) {
+            fence_async_smem();  // the row's copies went through the generic proxy (the copiers' own fence would drain their queue)
             fence_after();
-            issue_row<KC, COUT>(tmem, su32(ring + (a & 1) * L::IN_ROW), gy, su32(sm + L::OFF_W));
+            issue_row<KC, COUT>(tmem, su32(ring + a % L::NROW * L::IN_ROW), gy, su32(sm + L::OFF_W));
             commit(bar);
         }
-        if (a + 1 < nrows + 2) stage(gy + 1, (a + 1) & 1);  // its buffer was read by row a - 1's MMAs
+        // two rows ahead, into the buffer that row a - 1's MMAs read (an empty group keeps the count)
+        if (a + 2 < nrows + 2) stage(gy + 2, (a + 2) % L::NROW);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        // the mask of the output row that this input row completes, while the MMAs run
+        const int go = gy - 1, p = lane_q * 32 + lane, gx = x0 + p, c0 = half * HC;
+        const size_t cell = img_off + (size_t)go * W + gx;
+        const bool stored = go >= y0 && gx < W;
+        uint4 mk[HC / 8];
+        if (EPI == EPI_MASK && stored)
+#pragma unroll
+            for (int q = 0; q < HC / 8; ++q) mk[q] = reinterpret_cast<const uint4*>(mask + cell * COUT + c0)[q];
         if (tid == 0) s_ok = bar_wait_bounded(bar, parity) ? 1 : 0;
         __syncthreads();
         if (!s_ok) {
@@ -748,17 +777,13 @@ __global__ void __launch_bounds__(CONV_TC_THREADS, 4)
         parity ^= 1u;
         fence_after();
         // output row gy - 1 is complete; rows before y0 only had to be cleared
-        const int go = gy - 1;
         const int slot = ((go % 3) + 3) % 3;
         const unsigned t = tmem + lane_off + slot * COUT + half * HC;
-        const int p = lane_q * 32 + lane, gx = x0 + p;
         if (go >= y0) {
             float v[HC];
             if constexpr (HC == 16) tmem_ld16(t, v);
             else tmem_ld8(t, v);
-            if (gx < W) {
-                const size_t cell = img_off + (size_t)go * W + gx;
-                const int c0 = half * HC;
+            if (stored) {
                 if (EPI == EPI_BIAS_F32) {
                     float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + cell * COUT + c0);
 #pragma unroll
@@ -773,7 +798,6 @@ __global__ void __launch_bounds__(CONV_TC_THREADS, 4)
                             w[q] = pack_bf16x2(fmaxf(v[2 * q] + sbias[c0 + 2 * q], 0.0f),
                                                fmaxf(v[2 * q + 1] + sbias[c0 + 2 * q + 1], 0.0f));
                     } else {  // EPI_MASK
-                        const uint4* mk = reinterpret_cast<const uint4*>(mask + cell * COUT + c0);
 #pragma unroll
                         for (int q4 = 0; q4 < HC / 8; ++q4) {
                             const uint4 mm = mk[q4];
@@ -796,8 +820,7 @@ __global__ void __launch_bounds__(CONV_TC_THREADS, 4)
         if constexpr (HC == 16) tmem_zero16(t);
         else tmem_zero8(t);
         tmem_wait_st();
-        asm volatile("cp.async.wait_group 0;" ::: "memory");  // input row a + 1 landed
-        fence_async_smem();
+        asm volatile("cp.async.wait_group 1;" ::: "memory");  // input row a + 1 landed
         fence_before();
         __syncthreads();
     }

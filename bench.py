@@ -409,7 +409,9 @@ def run_gpu(args):
     bytes_per_cell = 18 * BYTES_PER_VALUE[args.dtype]
     achieved = bytes_per_cell * cells / per_launch_s / 1e9
     peak, peak_kind = measured_peak()
-    tr = committed_traffic(args)
+    # AUTO fuses FP32 steps: a launch moves a step's bytes for several of them
+    steps_per_launch = args.steps * len(ms_list) / max(1, gpu_launches)
+    tr = committed_traffic(args) if steps_per_launch <= 1.0 else None
 
     # ---- macro every step (the reference's behaviour), reported separately
     sim_m = FluidSimulator(macro_every_step=True, **params)
@@ -473,7 +475,10 @@ def run_gpu(args):
                          "frac": achieved / peak, "peak_source": peak_kind,
                          "traffic": (tr or {}).get("bytes_per_launch_scaled"),
                          "traffic_source": (tr or {}).get("source"),
-                         "algorithmic_bytes_per_launch": bytes_per_cell * cells},
+                         "algorithmic_bytes_per_launch": bytes_per_cell * cells,
+                         "steps_per_launch": steps_per_launch,
+                         "what": "achieved counts every step's populations once read and once written; "
+                                 "fused steps move them once per launch, so frac may exceed 1"},
             "macro_every_step_glups": glups_macro,
             "reference_mode_glups": glups_ref_mode.get("fast"),
             "reference_mode_exact_glups": glups_ref_mode.get("exact"),

@@ -414,6 +414,7 @@ int cluster_steps(const lbm_handle* h, int left) {
     int ready = 0;
     const cudaError_t e = h->p.collision == LBM_COLLISION_KBC ? cluster_ready<LBM_COLLISION_KBC>(h->device, &ready)
                                                               : cluster_ready<LBM_COLLISION_BGK>(h->device, &ready);
+    if (e != cudaSuccess) cudaGetLastError();  // not for the next launch's check
     if (e != cudaSuccess || ready < 1) return 1;
     return std::min(left, CL_MOST_STEPS);
 }

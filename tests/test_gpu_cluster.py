@@ -33,6 +33,8 @@ def _lattice(nx, ny, scene, block_iter=-1, far_outlet=False, **kw):
             info[ny // 2 - 2, nx // 2] = (6, block_iter, 0.01, -0.02)
         # moving obstacles, one beside the last column; a wall in that column, and a fluid cell across from it
         info[ny // 3, nx - 2] = info[ny // 4, nx // 3] = (4, -1, 0.02, -0.01)
+        if nx >= 64:  # inlets away from the first column, in both halves of a window
+            info[ny // 5, 5] = info[ny // 5, 40] = (3, -1, 0.02, 0.01)
         if scene == "channel":
             info[ny // 2, nx - 1] = info[2 * ny // 3, nx - 1] = (4, -1, 0.0, 0.01)
             info[ny // 2 - 1:ny // 2 + 2, 0] = (1, -1, 0.0, 0.0)

@@ -384,7 +384,7 @@ struct lbm_batch {
     lbm::BatchDomain* d_doms = nullptr;
     int4* d_tiles = nullptr;
     int ntiles = 0;
-    bool march = false;  // every domain fits the windows of k_batch_march
+    bool march = false;  // k_batch_march: every domain fits its windows, and there are cells enough
     int4* d_tasks = nullptr;
     int ntasks = 0, march_rows = 0;
     float* pool[2] = {nullptr, nullptr};
@@ -494,6 +494,11 @@ int with_form(const lbm_batch* b, F&& fn) {
         default: return fn(std::integral_constant<int, 4>{});
     }
 }
+
+// Cells from which a batch marches.  Below, a pass has fewer windows than warps and its time is that of
+// one window's rows (domains of the generator, GLUPS before and marching: 0.6 M cells 58 and 32, 1.0 M 73 and 55, 1.3 M
+// 71 and 62, 1.9 M 67 and 68, 3.2 M 71 and 78, 5.0 M 75 and 89).
+constexpr size_t BATCH_MARCH_CELLS = 2000000;
 
 // Rows of a task: whole waves of warps with little work done twice (T - 1 rows above and below a task
 // are computed for its first steps): the rows that minimise waves x (rows + halo).
@@ -758,8 +763,13 @@ int lbm_batch_create(int32_t n, const lbm_domain_desc* desc, lbm_batch** out) {
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    size_t domain_cells = 0;
     b->march = true;
-    for (const lbm::BatchDomain& dm : doms) b->march = b->march && dm.nx >= lbm::MARCH_W && dm.ny >= 8;
+    for (const lbm::BatchDomain& dm : doms) {
+        b->march = b->march && dm.nx >= lbm::MARCH_W && dm.ny >= 8;
+        domain_cells += (size_t)dm.nx * dm.ny;
+    }
+    b->march = b->march && domain_cells >= BATCH_MARCH_CELLS;
     int r = e == cudaSuccess ? build_tiles(b) : bfail(LBM_ERR_CUDA, "batch set-up: %s", cudaGetErrorString(e));
     if (r == LBM_OK && b->march) r = set_march_rows(b, march_rows_for(b));
     if (r != LBM_OK) {

@@ -11,7 +11,9 @@ pytestmark = pytest.mark.gpu
 
 DOMAINS = [dict(nx=64, ny=8, scene="cavity", tau=0.6, speed=0.08), dict(nx=65, ny=97, scene="channel", tau=0.7, speed=0.05),
            dict(nx=121, ny=64, scene="channel", tau=0.56, speed=0.03), dict(nx=257, ny=130, scene="cavity", tau=0.9, speed=0.1),
-           dict(nx=180, ny=201, scene="channel", tau=0.8, speed=0.07)]
+           dict(nx=180, ny=201, scene="channel", tau=0.8, speed=0.07),
+           # with this one the batch is large enough for fused steps
+           dict(nx=1500, ny=1400, scene="channel", tau=0.65, speed=0.06)]
 
 
 def test_fused_passes_equal_single_steps(gpu):

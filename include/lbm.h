@@ -403,8 +403,8 @@ int lbm_colorize(lbm_handle* h, int32_t mode, const float* d_curl, int32_t canva
    independent physics-mode FP32 lattices (moving-lid cavities and channels) of uneven
    size advance together: in one cooperative persistent launch per lbm_batch_step call,
    replayed from a CUDA graph (LBM_BATCH_PERSISTENT; up to three steps between grid barriers where
-   every domain is at least 64 x 8 cells, with the results of single steps bit for bit, and the
-   tile shapes below otherwise), in one tile-list launch per step
+   every domain is at least 64 x 8 cells and all together have two million, with the results of
+   single steps bit for bit, and the tile shapes below otherwise), in one tile-list launch per step
    (LBM_BATCH_TILE_LAUNCHES), or in one launch per domain and step
    (LBM_BATCH_DOMAIN_LOOP).  The persistent kernel's grid barrier waits at most a set time;
    a timed-out wait sets an error that lbm_batch_status returns as LBM_ERR_TIMEOUT.

@@ -365,10 +365,15 @@ int bfail(int code, const char* fmt, ...) {
         if (r_ < 0) return r_; \
     } while (0)
 
+// march: the batches that march have settings of their own (a batch of the same size with one domain too
+// narrow for a window does not)
 struct TuneKey {
     long cells_class;
-    int ndom;
-    bool operator<(const TuneKey& o) const { return std::tie(cells_class, ndom) < std::tie(o.cells_class, o.ndom); }
+    int ndom, device;
+    bool march;
+    bool operator<(const TuneKey& o) const {
+        return std::tie(cells_class, ndom, device, march) < std::tie(o.cells_class, o.ndom, o.device, o.march);
+    }
 };
 struct Tuned {
     lbm_batch_config cfg;
@@ -465,6 +470,7 @@ std::vector<int4> march_tasks(const lbm_batch* b, int rows) {
 }
 int set_march_rows(lbm_batch* b, int rows) {
     if (rows == b->march_rows) return LBM_OK;
+    if (rows < 1) return bfail(LBM_ERR_STATE, "tasks of %d rows", rows);  // (march_tasks walks down by them)
     const std::vector<int4> tasks = march_tasks(b, rows);
     if (b->d_tasks) cudaFree(b->d_tasks);
     b->d_tasks = nullptr;
@@ -879,7 +885,7 @@ int lbm_batch_tune(lbm_batch* b, int32_t trial_steps, lbm_batch_config* best_out
     B_TRY(check_batch(b));
     if (trial_steps < 1) return bfail(LBM_ERR_ARG, "trial_steps must be >= 1");
     B_CK(cudaSetDevice(b->device));
-    const TuneKey key{(long)std::lround(std::log2((double)b->live_cells + 1.0) * 4.0), (int)b->doms.size()};
+    const TuneKey key{(long)std::lround(std::log2((double)b->live_cells + 1.0) * 4.0), (int)b->doms.size(), b->device, b->march};
     auto it = g_tune_cache.find(key);
     if (it != g_tune_cache.end()) {
         B_TRY(lbm_batch_set_config(b, &it->second.cfg));
@@ -973,7 +979,7 @@ int lbm_batch_tune(lbm_batch* b, int32_t trial_steps, lbm_batch_config* best_out
         cudaEventDestroy(e1);
     }
     B_TRY(lbm_batch_set_config(b, &best));
-    g_tune_cache[key] = {best, b->march_rows};
+    g_tune_cache[key] = {best, march ? b->march_rows : 0};
     if (best_out) *best_out = best;
     return LBM_OK;
 }

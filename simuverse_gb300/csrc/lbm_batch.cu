@@ -36,6 +36,7 @@
 
 #include "lbm_cell4.cuh"
 #include "lbm_common.cuh"
+#include "lbm_device_list.h"
 #include "lbm_internal.h"
 #include "lbm_march.cuh"
 
@@ -381,17 +382,25 @@ struct Tuned {
 };
 std::map<TuneKey, Tuned> g_tune_cache;
 
+struct DeviceMem {
+    static constexpr cudaError_t OK = cudaSuccess;
+    static cudaError_t alloc(void** p, size_t bytes) { return cudaMalloc(p, bytes); }
+    static cudaError_t upload(void* dst, const void* src, size_t bytes) {
+        return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    }
+    static void release(void* p) { cudaFree(p); }
+};
+
 }  // namespace
 
 struct lbm_batch {
     std::vector<lbm_domain_desc> desc;
     std::vector<lbm::BatchDomain> doms;
     lbm::BatchDomain* d_doms = nullptr;
-    int4* d_tiles = nullptr;
-    int ntiles = 0;
+    lbm::DeviceList<int4, DeviceMem> tiles;
     bool march = false;  // k_batch_march: every domain fits its windows, and there are cells enough
-    int4* d_tasks = nullptr;
-    int ntasks = 0, march_rows = 0;
+    lbm::DeviceList<int4, DeviceMem> tasks;
+    int march_rows = 0;
     float* pool[2] = {nullptr, nullptr};
     uint16_t* d_flags = nullptr;
     lbm_lattice_info* d_info = nullptr;
@@ -431,11 +440,7 @@ int build_tiles(lbm_batch* b) {
         for (int y0 = 0; y0 < dm.ny; y0 += th)
             for (int x0 = 0; x0 < dm.pitch; x0 += tw) tiles.push_back(make_int4((int)d, x0, y0, 0));
     }
-    if (b->d_tiles) cudaFree(b->d_tiles);
-    b->d_tiles = nullptr;
-    B_CK(cudaMalloc((void**)&b->d_tiles, tiles.size() * sizeof(int4)));
-    B_CK(cudaMemcpy(b->d_tiles, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    b->ntiles = (int)tiles.size();
+    B_CK(b->tiles.replace(tiles));
     free_graph(b);
     return LBM_OK;
 }
@@ -471,15 +476,9 @@ std::vector<int4> march_tasks(const lbm_batch* b, int rows) {
 int set_march_rows(lbm_batch* b, int rows) {
     if (rows == b->march_rows) return LBM_OK;
     if (rows < 1) return bfail(LBM_ERR_STATE, "tasks of %d rows", rows);  // (march_tasks walks down by them)
-    const std::vector<int4> tasks = march_tasks(b, rows);
-    if (b->d_tasks) cudaFree(b->d_tasks);
-    b->d_tasks = nullptr;
-    b->march_rows = 0;
-    free_graph(b);
-    B_CK(cudaMalloc((void**)&b->d_tasks, tasks.size() * sizeof(int4)));
-    B_CK(cudaMemcpy(b->d_tasks, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    b->ntasks = (int)tasks.size();
+    B_CK(b->tasks.replace(march_tasks(b, rows)));
     b->march_rows = rows;
+    free_graph(b);
     return LBM_OK;
 }
 
@@ -568,15 +567,15 @@ int launch_persistent(lbm_batch* b, int nsteps, int skip_block, int skip_step, c
     lc.attrs = attr;
     lc.numAttrs = 1;
     if (b->march) {
-        B_CK(cudaLaunchKernelEx(&lc, lbm::k_batch_march, (const lbm::BatchDomain*)b->d_doms, (const int4*)b->d_tasks,
-                                b->ntasks, b->pool[0], b->pool[1], (const uint16_t*)b->d_flags,
+        B_CK(cudaLaunchKernelEx(&lc, lbm::k_batch_march, (const lbm::BatchDomain*)b->d_doms, (const int4*)b->tasks.data,
+                                b->tasks.count, b->pool[0], b->pool[1], (const uint16_t*)b->d_flags,
                                 (const lbm_lattice_info*)b->d_info, b->d_macro, nsteps, b->cur, macro, b->d_bar,
                                 b->timeout_ns, skip_block, skip_step));
         return LBM_OK;
     }
     B_TRY(with_form(b, [&](auto kf) {
         B_CK(cudaLaunchKernelEx(&lc, lbm::k_batch_persistent<decltype(kf)::value>, (const lbm::BatchDomain*)b->d_doms,
-                                (const int4*)b->d_tiles, b->ntiles, b->pool[0], b->pool[1], b->d_flags, b->d_info,
+                                (const int4*)b->tiles.data, b->tiles.count, b->pool[0], b->pool[1], b->d_flags, b->d_info,
                                 b->d_macro, nsteps, b->cur, b->d_bar, b->timeout_ns, skip_block, skip_step));
         return LBM_OK;
     }));
@@ -621,8 +620,8 @@ int run_steps(lbm_batch* b, int nsteps, int method) {
             const float* A = b->pool[(b->cur + s) & 1];
             float* B = b->pool[(b->cur + s + 1) & 1];
             B_TRY(with_form(b, [&](auto kf) {
-                lbm::k_batch_tiles<decltype(kf)::value><<<(unsigned)b->ntiles, block, 0, b->stream>>>(
-                    b->d_doms, b->d_tiles, A, B, b->d_flags, b->d_info, b->d_macro, s == nsteps - 1);
+                lbm::k_batch_tiles<decltype(kf)::value><<<(unsigned)b->tiles.count, block, 0, b->stream>>>(
+                    b->d_doms, b->tiles.data, A, B, b->d_flags, b->d_info, b->d_macro, s == nsteps - 1);
                 return LBM_OK;
             }));
             B_CK(cudaGetLastError());
@@ -799,8 +798,8 @@ int lbm_batch_destroy(lbm_batch* b) {
     cudaFree(b->d_part);
     cudaFree(b->d_bar);
     cudaFree(b->d_doms);
-    cudaFree(b->d_tiles);
-    cudaFree(b->d_tasks);
+    b->tiles.clear();
+    b->tasks.clear();
     if (b->own_stream) cudaStreamDestroy(b->own_stream);
     delete b;
     return LBM_OK;
@@ -840,8 +839,11 @@ int lbm_batch_set_config(lbm_batch* b, const lbm_batch_config* cfg) {
     B_CK(cudaStreamSynchronize(b->stream));
     const bool retile = tx != b->cfg.tile_threads_x || ty != b->cfg.tile_rows ||
                         cfg->cells_per_thread != b->cfg.cells_per_thread || cfg->linear != b->cfg.linear;
+    const lbm_batch_config before = b->cfg;
     b->cfg = *cfg;
-    if (retile) B_TRY(build_tiles(b));
+    const int r = retile ? build_tiles(b) : LBM_OK;
+    if (r != LBM_OK) b->cfg = before;  // the tile list is still that of the former shape
+    B_TRY(r);
     free_graph(b);
     return LBM_OK;
 }

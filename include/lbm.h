@@ -425,7 +425,8 @@ typedef struct lbm_domain_desc {
 typedef struct lbm_batch_config {
     int32_t tile_threads_x;   /* threads per tile row (multiple of 32) */
     int32_t tile_rows;        /* rows per tile (threads per block = tile_threads_x * tile_rows <= 256) */
-    int32_t blocks_per_sm;    /* persistent grid = blocks_per_sm x SMs (0: occupancy maximum) */
+    int32_t blocks_per_sm;    /* persistent grid = blocks_per_sm x SMs (0: occupancy maximum); fused steps
+                                 have a grid of their own */
     int32_t method;           /* LBM_BATCH_* */
     float ms_per_step;        /* filled by lbm_batch_tune */
     int32_t cells_per_thread; /* 1, or 4 (vector accesses); a tile is cells_per_thread * tile_threads_x wide */
@@ -449,7 +450,9 @@ int lbm_batch_info(const lbm_batch* b, int32_t* ndomains, uint64_t* cells);
 int lbm_batch_set_config(lbm_batch* b, const lbm_batch_config* cfg);
 int lbm_batch_get_config(const lbm_batch* b, lbm_batch_config* cfg);
 /* times trial_steps of every candidate tile shape and grid size, keeps the fastest
-   (cached per shape class for the life of the process) */
+   (cached per shape class for the life of the process).  A batch that takes fused steps keeps the
+   fastest height of their windows as well; that is no field of the configuration, so a saved one
+   brings it back only through this call. */
 int lbm_batch_tune(lbm_batch* b, int32_t trial_steps, lbm_batch_config* best);
 int lbm_batch_step(lbm_batch* b, int32_t nsteps);
 /* synchronises; LBM_ERR_TIMEOUT if a persistent launch's grid barrier timed out */

@@ -524,9 +524,10 @@ int march_rows_for(const lbm_batch* b) {
     return rows;
 }
 
+// Blocks of a persistent launch.  cfg.blocks_per_sm is a choice for the tile kernels (the tuner's best of 2 to 16);
+// the march takes what it is compiled for: with two blocks for three it would run on two thirds of its warps.
 int persistent_grid(lbm_batch* b, int* grid) {
     int per_sm = 0;
-    const int threads = b->march ? 32 * lbm::BM_WARPS : b->cfg.tile_threads_x * b->cfg.tile_rows;
     if (b->march) {
         constexpr int SMEM = lbm::BM_WARPS * lbm::march_smem(3);
         static lbm::PerDevice<int> fit;
@@ -539,7 +540,11 @@ int persistent_grid(lbm_batch* b, int* grid) {
                                                                                         32 * lbm::BM_WARPS, SMEM);
             },
             &per_sm));
-    } else
+        if (per_sm < 1) return bfail(LBM_ERR_CUDA, "the kernel of fused steps does not fit the device");
+        *grid = per_sm * b->sms;
+        return LBM_OK;
+    }
+    const int threads = b->cfg.tile_threads_x * b->cfg.tile_rows;
     B_TRY(with_form(b, [&](auto kf) {
         B_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lbm::k_batch_persistent<decltype(kf)::value>,
                                                            threads, 0));
@@ -951,12 +956,13 @@ int lbm_batch_tune(lbm_batch* b, int32_t trial_steps, lbm_batch_config* best_out
                 }
             }
         }
-    if (march) {
+    int r = lbm_batch_set_config(b, &best);
+    if (march && r == LBM_OK) {
         // the rows of a task, timed on single passes from the current pool into the other one, which
         // leave the state where it is
         b->march = true;
         best_ms = 1e30f;
-        int best_rows = b->march_rows, r = LBM_OK;
+        int best_rows = b->march_rows;
         for (int rows : {march_rows_for(b), 16, 24, 32, 48}) {
             float ms = 0.0f;
             if (r == LBM_OK) r = set_march_rows(b, rows);
@@ -972,15 +978,11 @@ int lbm_batch_tune(lbm_batch* b, int32_t trial_steps, lbm_batch_config* best_out
             }
         }
         if (r == LBM_OK) r = set_march_rows(b, best_rows);
-        best.ms_per_step = best_ms;
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        B_TRY(r);
-    } else {
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
+        b->cfg.ms_per_step = best.ms_per_step = best_ms;
     }
-    B_TRY(lbm_batch_set_config(b, &best));
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    B_TRY(r);
     g_tune_cache[key] = {best, march ? b->march_rows : 0};
     if (best_out) *best_out = best;
     return LBM_OK;

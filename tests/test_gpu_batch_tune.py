@@ -46,3 +46,30 @@ def test_two_batches_of_one_class(gpu, first, second, others):
         _check(c, domains)
         for x in (b, c):
             x.close()
+
+
+def test_fused_steps_have_a_grid_of_their_own(gpu):
+    """A tile form of one block per SM does not take warps from the fused steps: a block of the second half of their
+    grid exists, and its absence is noticed."""
+    import torch
+
+    from simuverse_gb300 import _native as nat
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    b = BatchSimulator([WIDE, BIG])
+    b.configure(blocks_per_sm=1)
+    assert b.inject_missing_arrival(nsteps=7, block=2 * sms, step=4, timeout_ns=200_000_000) == nat.LBM_ERR_TIMEOUT
+    b.close()
+    # and the time reported is that of the setting that runs: at most a few times the time of a long call
+    b = BatchSimulator([WIDE, BIG, MORE, MORE])
+    ms = b.tune(trial_steps=3)["ms_per_step"]
+    e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    stream = torch.cuda.Stream()
+    b.set_stream(stream.cuda_stream)
+    b.step(300)
+    e[0].record(stream)
+    b.step(300)
+    e[1].record(stream)
+    stream.synchronize()
+    assert e[0].elapsed_time(e[1]) / 300 <= 1.5 * ms
+    b.close()

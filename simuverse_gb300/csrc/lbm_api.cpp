@@ -492,6 +492,76 @@ int sync(lbm_handle* h) {
     return LBM_OK;
 }
 
+// Scratch of the handle's stream: from the pool, or page-locked host memory (which kernels reach as well) where
+// the device has none left, so that an edit of a lattice that fills it still works.  The bounds-checked build
+// takes the second way always, so that it is tested.
+struct Scratch {
+    void* p = nullptr;
+    bool host = false;
+    cudaError_t get(size_t bytes, cudaStream_t s) {
+#ifdef LBM_BOUNDS_CHECK
+        cudaError_t e = cudaErrorMemoryAllocation;
+#else
+        cudaError_t e = pool_alloc(&p, bytes, s);
+#endif
+        if (e != cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();  // not for the next launch's check
+        host = true;
+        return cudaHostAlloc(&p, bytes, cudaHostAllocDefault);
+    }
+    void release(cudaStream_t s) {
+        if (!host) return pool_free(p, s);
+        cudaStreamSynchronize(s);
+        if (p) cudaFreeHost(p);
+    }
+};
+
+// Brings the other buffer from what the last launch of several steps read to what single steps leave there,
+// the state one step before the current one.  It is called before anything that makes the other buffer's content
+// last: a cell that turns solid keeps it (ring cells of the reference's rules pull from it, and it is there
+// when the cell turns fluid again), checkpoints hold both buffers, and an initialisation leaves fluid cells of one
+// as they are.  A launch of several steps computes with records and flags that do not change, so its
+// steps can be taken again.  Asynchronous on the handle's stream.
+int catch_up(lbm_handle* h) {
+    if (h->behind < 2) return LBM_OK;
+    const int n = h->behind - 1, cur = h->cur;
+    void* const now = h->buf[cur];
+    void* const old = h->buf[cur ^ 1];
+    const float omega = h->omega;
+    const size_t bytes = 9 * h->N * lbm::dtype_size(h->p.dtype);
+    cudaError_t e = cudaSuccess;
+    h->omega = h->behind_omega;
+    if (h->behind_cluster) {
+        h->buf[cur] = h->buf[cur ^ 1] = old;
+        e = lbm::launch_cluster(h, n, false, h->stream);
+    } else {
+        // One or two single steps through scratch.  Its solid cells' slots are those of the buffer that single steps
+        // would have had there: of two steps the current one's (the reference's rules read them), else the
+        // other one's, which agree and come back with the copy.
+        Scratch tmp;
+        e = tmp.get(bytes, h->stream);
+        if (e == cudaSuccess && (n == 1 || h->p.mode == LBM_MODE_REFERENCE))
+            e = cudaMemcpyAsync(tmp.p, n == 1 ? old : now, bytes, cudaMemcpyDefault, h->stream);
+        h->buf[cur] = old;
+        h->buf[cur ^ 1] = tmp.p;
+        if (e == cudaSuccess) e = lbm::launch_step(h, false, h->stream);
+        if (n == 1) {
+            if (e == cudaSuccess) e = cudaMemcpyAsync(old, tmp.p, bytes, cudaMemcpyDefault, h->stream);
+        } else {
+            std::swap(h->buf[0], h->buf[1]);
+            if (e == cudaSuccess) e = lbm::launch_step(h, false, h->stream);
+        }
+        tmp.release(h->stream);
+    }
+    h->buf[cur] = now;
+    h->buf[cur ^ 1] = old;
+    h->omega = omega;
+    if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "steps taken again: %s", cudaGetErrorString(e));
+    h->launches += h->behind_cluster ? 1 : n;
+    h->behind = 1;
+    return LBM_OK;
+}
+
 // the lattice's buffers back to the pool (ordered on the lattice's own stream: the caller has
 // waited for the stream the lattice ran on)
 void free_all(lbm_handle* h) {
@@ -694,7 +764,7 @@ int lbm_step(lbm_handle* h, int32_t nsteps) {
         if (small > 1) LBM_CK(lbm::launch_cluster(h, n, macro, h->stream));
         else LBM_CK(n > 1 ? lbm::launch_fused(h, n, macro, h->stream) : lbm::launch_step(h, macro, h->stream));
         s += n;
-        h->cur ^= small > 1 ? n & 1 : 1;
+        lbm::took_steps(h, n, small > 1);
         h->steps += n;
         h->countdown = std::max<int64_t>(0, h->countdown - n);
         ++h->launches;
@@ -709,6 +779,7 @@ int lbm_reset(lbm_handle* h) {
     LbmRange range_("lbm_reset");
     LBM_TRY(check_handle(h));
     LBM_TRY(use_device(h));
+    LBM_TRY(catch_up(h));
     // reference: only the Poiseuille scene rebuilds its mask (d2q9_node.rs:248-255)
     int r = LBM_OK;
     if (device_scene(h->p)) {
@@ -753,6 +824,7 @@ int lbm_add_obstacle(lbm_handle* h, int32_t x, int32_t y) {
     if (x < 0 || x >= h->nx || min_y < 0 || max_y > h->ny)
         return fail(LBM_ERR_ARG, "obstacle rows [%d, %d) or column %d outside the lattice", min_y, max_y, x);
     LBM_TRY(use_device(h));
+    LBM_TRY(catch_up(h));
     ensure_host_info(h);
     h->no_solids = h->solids_agree = false;
     restart_countdown(h, min_y, max_y);
@@ -882,6 +954,7 @@ int lbm_apply_edits(lbm_handle* h, const lbm_edit* edits, int32_t n, int32_t* ap
         }
     }
     LBM_TRY(use_device(h));
+    if (!obs.empty()) LBM_TRY(catch_up(h));
     // a cell written by several strokes keeps the last one
     if (forces.size() > 1) {
         std::vector<size_t> order(forces.size());
@@ -983,6 +1056,7 @@ int lbm_set_info(lbm_handle* h, const lbm_lattice_info* info) {
     LBM_TRY(check_handle(h));
     if (!info) return fail(LBM_ERR_ARG, "null info");
     LBM_TRY(use_device(h));
+    LBM_TRY(catch_up(h));
     h->host_info.assign(info, info + h->N);
     h->host_info_lazy = false;
     h->no_solids = false;
@@ -1054,6 +1128,7 @@ int lbm_write_populations(lbm_handle* h, const void* src, int32_t sd) {
     if (!src) return fail(LBM_ERR_ARG, "null input");
     if (sd != LBM_DTYPE_F32 && sd != LBM_DTYPE_F64) return fail(LBM_ERR_ARG, "write dtype must be F32 or F64");
     LBM_TRY(use_device(h));
+    LBM_TRY(catch_up(h));  // which may need the current buffer's walls
     const size_t bytes = 9 * h->N * lbm::dtype_size(sd);
     void* tmp = nullptr;
     LBM_CK(pool_alloc(&tmp, bytes, h->stream));
@@ -1075,6 +1150,7 @@ int lbm_init_equilibrium(lbm_handle* h, const float* rho, const float* ux, const
     LBM_TRY(check_handle(h));
     if (h->p.mode != LBM_MODE_PHYSICS) return fail(LBM_ERR_STATE, "equilibrium initialisation is a physics-mode call");
     LBM_TRY(use_device(h));
+    LBM_TRY(catch_up(h));
     float* d = nullptr;
     const size_t plane = h->N * sizeof(float);
     LBM_CK(pool_alloc(&d, 3 * plane, h->stream));
@@ -1154,6 +1230,7 @@ int lbm_save(lbm_handle* h, const char* path) {
     LBM_TRY(check_handle(h));
     if (!path) return fail(LBM_ERR_ARG, "null path");
     LBM_TRY(use_device(h));
+    LBM_TRY(catch_up(h));
     LBM_TRY(sync(h));
     const size_t pop_bytes = 9 * h->N * lbm::dtype_size(h->p.dtype);
     std::vector<char> state(2 * pop_bytes);
@@ -1226,6 +1303,7 @@ int lbm_load(lbm_handle* h, const char* path) {
     lbm::cluster_cells(h, info.data(), false);
     lbm::cluster_cells(h, hinfo.data(), true);  // its rows may be uploaded
     h->no_solids = h->solids_agree = false;
+    h->behind = 1;
     h->cur = hd.cur & 1;
     h->tau = hd.tau;
     h->omega = 1.0f / hd.tau;

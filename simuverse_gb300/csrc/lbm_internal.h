@@ -8,6 +8,7 @@
 
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/lbm.h"
@@ -56,6 +57,11 @@ struct lbm_handle {
     // writes hold the same in both buffers
     int64_t countdown = 0;
     bool no_solids = false, solids_agree = false;
+    // what the other buffer holds: the state `behind` steps before the current one.  Single steps leave 1; the
+    // last launch of several steps (a cluster's or a march) leaves their number, computed at rate behind_omega
+    int behind = 1;
+    bool behind_cluster = false;
+    float behind_omega = 0.0f;
     // and what those of small lattices ask (lbm_step_cluster.cu): no outflow cell outside the last column; any
     // inlet or outflow cell
     bool outlets_last = true, faces = false;
@@ -146,10 +152,22 @@ cudaError_t launch_ref_init(lbm_handle* h, cudaStream_t s);
 cudaError_t launch_phys_init(lbm_handle* h, const float* d_rho, const float* d_ux, const float* d_uy,
                              cudaStream_t s);
 cudaError_t launch_step(lbm_handle* h, bool write_macro, cudaStream_t s);
+// A launch of several steps reads buffer cur and writes the other one.  An odd number leaves every solid
+// cell's slots where single steps would; an even number does if the two buffers agree there.
+inline bool even_steps(const lbm_handle* h) { return h->no_solids || h->solids_agree; }
+// After such a launch: the state is in the other buffer.  Single steps leave it in `cur` again after an even
+// number, so the buffers change their names there and `cur` stays (it goes into checkpoints).
+inline void took_steps(lbm_handle* h, int n, bool cluster) {
+    if (n & 1) h->cur ^= 1;
+    else std::swap(h->buf[0], h->buf[1]);
+    h->behind = n;
+    h->behind_cluster = cluster;
+    h->behind_omega = h->omega;
+}
 // fused steps (lbm_step_fused.cu): how many of the next `left` steps one launch takes (1: launch_step)
 int fused_steps(const lbm_handle* h, int left);
 cudaError_t launch_fused(lbm_handle* h, int steps, bool write_macro, cudaStream_t s);
-// the same for a small lattice (lbm_step_cluster.cu): the state ends in buffer cur ^ (steps & 1)
+// the same for a small lattice (lbm_step_cluster.cu); the buffers may be one (the launch reads all of it first)
 int cluster_steps(const lbm_handle* h, int left);
 cudaError_t launch_cluster(lbm_handle* h, int steps, bool write_macro, cudaStream_t s);
 // h->outlets_last and h->faces of the records of a lattice small enough for it (also: and of those seen before)

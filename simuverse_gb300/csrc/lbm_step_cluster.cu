@@ -416,13 +416,14 @@ int cluster_steps(const lbm_handle* h, int left) {
                                                               : cluster_ready<LBM_COLLISION_BGK>(h->device, &ready);
     if (e != cudaSuccess) cudaGetLastError();  // not for the next launch's check
     if (e != cudaSuccess || ready < 1) return 1;
-    return std::min(left, CL_MOST_STEPS);
+    const int n = std::min(left, CL_MOST_STEPS);
+    return n % 2 == 1 || even_steps(h) ? n : n - 1;
 }
 
 template <int COLL>
 static cudaError_t cluster_c(lbm_handle* h, int steps, bool macro, cudaStream_t s) {
-    // the state ends in the buffer where single steps would leave it; solid cells' slots are not written
-    const FusedLattice L = {(const float*)h->buf[h->cur], (float*)h->buf[h->cur ^ (steps & 1)], h->d_flags, h->d_info,
+    // (solid cells' slots are not written)
+    const FusedLattice L = {(const float*)h->buf[h->cur], (float*)h->buf[h->cur ^ 1], h->d_flags, h->d_info,
                             h->d_macro, h->nx, h->nx, h->ny, (uint32_t)h->N};
     ClusterShape shape;
     shape.windows = cluster_windows(h->nx);

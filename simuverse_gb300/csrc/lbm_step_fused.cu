@@ -60,9 +60,7 @@ int fused_steps(const lbm_handle* h, int left) {
         h->nx < MARCH_W || h->ny < 8 || h->N < FUSED_CELLS)
         return 1;
     if (h->p.mode == LBM_MODE_PHYSICS ? !core_has(h->p.collision) : h->p.arith != LBM_ARITH_FAST) return 1;
-    // A launch swaps the buffers once.  An odd number of steps leaves every solid cell's slots where
-    // single steps would; an even number needs the two buffers to agree there.
-    const bool even = h->no_solids || h->solids_agree;
+    const bool even = even_steps(h);
     if (left >= 3 && !(left == 4 && even)) return 3;
     return left >= 2 && even ? 2 : 1;
 }
@@ -90,7 +88,7 @@ static cudaError_t march_launch(PerDevice<int>& setup, K* kernel, const C& k, lb
     // without solids 4 % slower in eight than in two to four.
     const int windows = (h->nx + MARCH_OUT - 1) / MARCH_OUT;
     const long slots = (long)sms * MARCH_BLOCKS;
-        int rows = std::max(24, (int)((long)h->ny * windows / (slots * 8)));
+    int rows = std::max(24, (int)((long)h->ny * windows / (slots * 8)));
     const long waves = ((long)windows * ((h->ny + rows - 1) / rows) + slots - 1) / slots;
     if (waves < 4) {
         const long most = std::max(1L, waves * slots / windows);

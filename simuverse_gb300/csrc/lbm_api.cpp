@@ -477,13 +477,20 @@ void restart_countdown(lbm_handle* h, int y0, int y1) {
     const lbm_lattice_info* rows = h->host_info.data() + (size_t)y0 * h->nx;
     h->countdown = std::max(h->countdown, longest_countdown(rows, (size_t)(y1 - y0) * h->nx));
 }
-// the same over the device's records, which were all replaced; waits for the stream
-int whole_countdown(lbm_handle* h) {
-    unsigned long long n = 0;
+// The same over the device's records, which were all replaced, and whether the walls' slots that no step writes
+// hold the same in both buffers (a new solid cell keeps what it held as fluid, another step in each; new
+// velocities change nothing).  Waits for the stream.
+int recount(lbm_handle* h) {
+    unsigned long long n = 0, differ = 1;
     LBM_CK(lbm::launch_longest_countdown(h, h->stream));
     LBM_CK(cudaMemcpyAsync(&n, h->d_count, sizeof(n), cudaMemcpyDeviceToHost, h->stream));
+    if (h->p.dtype == LBM_DTYPE_F32 && h->p.kernel == LBM_KERNEL_AUTO) {  // the others take single steps
+        LBM_CK(lbm::launch_count_solid_slots(h, h->stream));
+        LBM_CK(cudaMemcpyAsync(&differ, h->d_count, sizeof(differ), cudaMemcpyDeviceToHost, h->stream));
+    }
     LBM_CK(cudaStreamSynchronize(h->stream));
     h->countdown = (int64_t)n;
+    h->solids_agree = differ == 0;
     return LBM_OK;
 }
 
@@ -1060,12 +1067,12 @@ int lbm_set_info(lbm_handle* h, const lbm_lattice_info* info) {
     h->host_info.assign(info, info + h->N);
     h->host_info_lazy = false;
     h->no_solids = false;
-    h->solids_agree = false;  // a new solid cell keeps what it held as fluid, another step in each buffer
+    h->solids_agree = false;
     h->countdown = INT64_MAX;
     lbm::cluster_cells(h, info, false);
     LBM_TRY(upload_info_rows(h, 0, h->ny));
     LBM_TRY(rebuild_flags(h));
-    return whole_countdown(h);
+    return recount(h);
 }
 
 int lbm_get_info(lbm_handle* h, lbm_lattice_info* out) {
@@ -1315,7 +1322,7 @@ int lbm_load(lbm_handle* h, const char* path) {
     h->p.scene = hd.scene;
     h->fluid_ty = hd.fluid_ty;
     LBM_TRY(rebuild_flags(h));
-    return whole_countdown(h);
+    return recount(h);
 }
 
 int lbm_status(lbm_handle* h) {

@@ -115,6 +115,29 @@ def test_what_else_keeps_the_other_buffer(gpu, tmp_path, size, scene, form, n):
         _same(*pair, "reset")
 
 
+@pytest.mark.parametrize("scene,form", [("custom", dict(mode="reference", arith="fast")), ("cavity", dict(mode="physics"))])
+def test_unlike_walls_do_not_outlive_their_cause(gpu, tmp_path, scene, form):
+    """New records that leave the walls as they were, and a checkpoint of a lattice whose walls agree: a frame of two
+    steps is one launch."""
+    a, b = _pair(LARGE, scene, form)
+    _both((a, b), lambda s: s.step(3))
+    info = a.info()
+    info["vx"][5, 5] = 0.01
+    _both((a, b), lambda s: s.set_info(info))
+    before = a.kernel_launches
+    _both((a, b), lambda s: s.compute())
+    assert a.kernel_launches == before + 1
+    _same(a, b, "records")
+    path = str(tmp_path / "walls")
+    b.save(path)
+    c = _pair(LARGE, scene, form)[0]
+    c.load(path)
+    before = c.kernel_launches
+    _both((c, b), lambda s: s.compute())
+    assert c.kernel_launches == before + 1
+    _same(c, b, "checkpoint")
+
+
 def child_main():
     import ctypes
 

@@ -198,7 +198,9 @@ int lbm_memory_set_retain(uint64_t bytes);
 int lbm_memory_trim(void);
 int lbm_memory_stats(uint64_t* reserved, uint64_t* used);
 /* run the handle's work on a caller-owned cudaStream_t (NULL restores its own stream);
-   no counterpart in the reference */
+   no counterpart in the reference.  lbm_step may be captured into a graph there; replays stay in order with
+   plain calls if the captured number of steps is even (an odd one ends in the other buffer).  A lattice
+   whose steps were captured takes one step per launch from then on. */
 int lbm_set_stream(lbm_handle* h, void* cuda_stream);
 int lbm_get_size(const lbm_handle* h, int32_t* nx, int32_t* ny);
 int lbm_get_params(const lbm_handle* h, lbm_params* out);

@@ -764,16 +764,23 @@ int lbm_step(lbm_handle* h, int32_t nsteps) {
     LBM_TRY(check_handle(h));
     if (nsteps < 0) return fail(LBM_ERR_ARG, "negative step count");
     LBM_TRY(use_device(h));
+    // A graph that holds captured steps reads and writes the buffers by address, at times that only its owner knows: a
+    // lattice whose steps were captured once takes single steps from then on.  They leave the state where a replay
+    // looks for it, leave the other buffer one step back, and heed records that count down, set before a replay or after.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &capture) != cudaSuccess) cudaGetLastError();
+    const bool capturing = capture != cudaStreamCaptureStatusNone;
+    h->captured |= capturing;
     for (int32_t s = 0; s < nsteps;) {
-        const int small = lbm::cluster_steps(h, nsteps - s);
-        const int n = small > 1 ? small : lbm::fused_steps(h, nsteps - s);
+        const int small = h->captured ? 1 : lbm::cluster_steps(h, nsteps - s);
+        const int n = h->captured ? 1 : (small > 1 ? small : lbm::fused_steps(h, nsteps - s));
         const bool macro = h->p.macro_every_step || s + n == nsteps;
         if (small > 1) LBM_CK(lbm::launch_cluster(h, n, macro, h->stream));
         else LBM_CK(n > 1 ? lbm::launch_fused(h, n, macro, h->stream) : lbm::launch_step(h, macro, h->stream));
         s += n;
         lbm::took_steps(h, n, small > 1);
         h->steps += n;
-        h->countdown = std::max<int64_t>(0, h->countdown - n);
+        if (!capturing) h->countdown = std::max<int64_t>(0, h->countdown - n);
         ++h->launches;
     }
     if (nsteps > 0) h->stepped_since_init = true;

@@ -62,6 +62,7 @@ struct lbm_handle {
     int behind = 1;
     bool behind_cluster = false;
     float behind_omega = 0.0f;
+    bool captured = false;  // a graph of the caller's holds steps: see lbm_step
     // and what those of small lattices ask (lbm_step_cluster.cu): no outflow cell outside the last column; any
     // inlet or outflow cell
     bool outlets_last = true, faces = false;

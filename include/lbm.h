@@ -404,9 +404,10 @@ int lbm_colorize(lbm_handle* h, int32_t mode, const float* d_curl, int32_t canva
    Batched form -- no counterpart in the reference (simuverse runs one lattice).  Many
    independent physics-mode FP32 lattices (moving-lid cavities and channels) of uneven
    size advance together: in one cooperative persistent launch per lbm_batch_step call,
-   replayed from a CUDA graph (LBM_BATCH_PERSISTENT; up to three steps between grid barriers where
-   every domain is at least 64 x 8 cells and all together have two million, with the results of
-   single steps bit for bit, and the tile shapes below otherwise), in one tile-list launch per step
+   replayed from a CUDA graph (LBM_BATCH_PERSISTENT; calls of three steps or more take up to three between
+   grid barriers, with the results of single steps bit for bit, where that is the faster form: every
+   domain at least 64 x 8 cells, all together two million, widths that fill windows of 60 columns; the
+   tile shapes below otherwise), in one tile-list launch per step
    (LBM_BATCH_TILE_LAUNCHES), or in one launch per domain and step
    (LBM_BATCH_DOMAIN_LOOP).  The persistent kernel's grid barrier waits at most a set time;
    a timed-out wait sets an error that lbm_batch_status returns as LBM_ERR_TIMEOUT.
@@ -452,9 +453,9 @@ int lbm_batch_info(const lbm_batch* b, int32_t* ndomains, uint64_t* cells);
 int lbm_batch_set_config(lbm_batch* b, const lbm_batch_config* cfg);
 int lbm_batch_get_config(const lbm_batch* b, lbm_batch_config* cfg);
 /* times trial_steps of every candidate tile shape and grid size, keeps the fastest
-   (cached per shape class for the life of the process).  A batch that takes fused steps keeps the
-   fastest height of their windows as well; that is no field of the configuration, so a saved one
-   brings it back only through this call. */
+   (cached per shape class for the life of the process).  Whether a batch takes fused steps, and the
+   height of their windows, are timed as well; they are no field of the configuration, so a batch that
+   is given a saved one has them by rule. */
 int lbm_batch_tune(lbm_batch* b, int32_t trial_steps, lbm_batch_config* best);
 int lbm_batch_step(lbm_batch* b, int32_t nsteps);
 /* synchronises; LBM_ERR_TIMEOUT if a persistent launch's grid barrier timed out */

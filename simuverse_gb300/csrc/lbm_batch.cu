@@ -12,7 +12,7 @@
 // tile at a domain's right edge; a tile list covers them all (one cell per thread, or four
 // with vector accesses).
 // Method 0: one cooperative persistent launch runs every step: warps take windows of a domain for
-// up to three fused steps (k_batch_march), or, where a domain is too small for them, blocks take tiles
+// up to three fused steps (k_batch_march), or, where that does not pay (march_share), blocks take tiles
 // round-robin for one step; then they meet at a grid barrier.  The barrier spins with
 // a time limit: a block that waits longer sets an error word (LBM_ERR_TIMEOUT), every
 // waiting block sees it and leaves, and the host reads the status -- no trap, the context
@@ -366,19 +366,18 @@ int bfail(int code, const char* fmt, ...) {
         if (r_ < 0) return r_; \
     } while (0)
 
-// march: the batches that march have settings of their own (a batch of the same size with one domain too
-// narrow for a window does not)
+// march: batches that may march have settings of their own, by the share of their work (march_share; a batch of the
+// same size with one domain too narrow for a window may not: 0)
 struct TuneKey {
     long cells_class;
-    int ndom, device;
-    bool march;
+    int ndom, device, march;
     bool operator<(const TuneKey& o) const {
         return std::tie(cells_class, ndom, device, march) < std::tie(o.cells_class, o.ndom, o.device, o.march);
     }
 };
 struct Tuned {
     lbm_batch_config cfg;
-    int rows;  // of a task of k_batch_march, 0 where it does not apply
+    int rows;  // of a task of k_batch_march, 0 for the tile form
 };
 std::map<TuneKey, Tuned> g_tune_cache;
 
@@ -398,7 +397,8 @@ struct lbm_batch {
     std::vector<lbm::BatchDomain> doms;
     lbm::BatchDomain* d_doms = nullptr;
     lbm::DeviceList<int4, DeviceMem> tiles;
-    bool march = false;  // k_batch_march: every domain fits its windows, and there are cells enough
+    bool can_march = false;  // every domain fits the windows of k_batch_march, and there are cells enough
+    bool march = false;      // and it is the faster form, by march_share or by lbm_batch_tune
     lbm::DeviceList<int4, DeviceMem> tasks;
     int march_rows = 0;
     float* pool[2] = {nullptr, nullptr};
@@ -500,7 +500,7 @@ int with_form(const lbm_batch* b, F&& fn) {
     }
 }
 
-// Cells from which a batch marches.  Below, a pass has fewer windows than warps and its time is that of
+// Cells from which a batch may march.  Below, a pass has fewer windows than warps and its time is that of
 // one window's rows (domains of the generator, GLUPS before and marching: 0.6 M cells 58 and 32, 1.0 M 73 and 55, 1.3 M
 // 71 and 62, 1.9 M 67 and 68, 3.2 M 71 and 78, 5.0 M 75 and 89).
 constexpr size_t BATCH_MARCH_CELLS = 2000000;
@@ -524,11 +524,36 @@ int march_rows_for(const lbm_batch* b) {
     return rows;
 }
 
+// Marching pays where enough of a pass's work becomes stored cells.  What does not: windows that a domain's width
+// does not fill, first and last windows (their rows take about 1.5 times an inner one's at walls, 2.2 times at
+// inlets and outflows), five rows of a task that are computed for its neighbours, and a last wave of tasks that is
+// not full.  Equal domains, that share and the time a step of the tile form over that of the march, both tuned:
+// 64^2 0.26 and 0.90 (cavities), 0.17 and 0.53 (channels); 64 x 128 channels 0.19 and 0.57; 121 x 300 0.44 and
+// 0.93; 200 x 110 0.56 and 1.01, channels 0.44 and 0.85; 181^2 0.49 and 0.84; 300 x 200 0.68 and 1.25, channels
+// 0.55 and 1.06; 500^2 0.69 and 1.15, channels 0.61 and 0.94; 1000 x 700 0.78 and 1.34, channels 0.73 and 1.04;
+// domains of the generator 0.65 to 0.72 and 1.10 to 1.45.
+double march_share(const lbm_batch* b, int rows) {
+    double work = 0.0, tasks = 0.0;
+    for (const lbm::BatchDomain& dm : b->doms) {
+        const double windows = (dm.nx + lbm::MARCH_OUT - 1) / lbm::MARCH_OUT, segments = (dm.ny + rows - 1) / rows;
+        const double edge = dm.scene == LBM_SCENE_CAVITY ? 1.5 : 2.2;
+        work += (windows + (edge - 1.0) * std::min(windows, 2.0)) * (dm.ny + 5.0 * segments);
+        tasks += windows * segments;
+    }
+    const double waves = tasks / ((double)b->sms * lbm::BM_BLOCKS * lbm::BM_WARPS);
+    if (waves > 1.0) work *= std::ceil(waves) / waves;
+    return (double)b->live_cells / (lbm::MARCH_OUT * work);
+}
+constexpr double MARCH_SHARE = 0.64;
+// Whether a persistent call of nsteps marches.  One or two steps are one pass, whose reads and writes they hardly
+// share: 0.5 to 0.75 and 0.55 to 0.95 times as fast as the tile form over the domains above.
+bool marches(const lbm_batch* b, int nsteps) { return b->march && nsteps >= 3; }
+
 // Blocks of a persistent launch.  cfg.blocks_per_sm is a choice for the tile kernels (the tuner's best of 2 to 16);
 // the march takes what it is compiled for: with two blocks for three it would run on two thirds of its warps.
-int persistent_grid(lbm_batch* b, int* grid) {
+int persistent_grid(lbm_batch* b, bool march, int* grid) {
     int per_sm = 0;
-    if (b->march) {
+    if (march) {
         constexpr int SMEM = lbm::BM_WARPS * lbm::march_smem(3);
         static lbm::PerDevice<int> fit;
         B_CK(fit.get(
@@ -558,20 +583,21 @@ int persistent_grid(lbm_batch* b, int* grid) {
 
 int launch_persistent(lbm_batch* b, int nsteps, int skip_block, int skip_step, cudaStream_t s, bool macro = true) {
     int grid = 0;
-    B_TRY(persistent_grid(b, &grid));
+    const bool march = marches(b, nsteps);
+    B_TRY(persistent_grid(b, march, &grid));
     B_CK(cudaMemsetAsync(b->d_bar, 0, sizeof(lbm::BarrierState), s));
     cudaLaunchConfig_t lc;
     std::memset(&lc, 0, sizeof(lc));
     lc.gridDim = dim3((unsigned)grid);
-    lc.blockDim = b->march ? dim3(32u * lbm::BM_WARPS) : dim3((unsigned)b->cfg.tile_threads_x, (unsigned)b->cfg.tile_rows);
-    lc.dynamicSmemBytes = b->march ? lbm::BM_WARPS * lbm::march_smem(3) : 0;
+    lc.blockDim = march ? dim3(32u * lbm::BM_WARPS) : dim3((unsigned)b->cfg.tile_threads_x, (unsigned)b->cfg.tile_rows);
+    lc.dynamicSmemBytes = march ? lbm::BM_WARPS * lbm::march_smem(3) : 0;
     lc.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     lc.attrs = attr;
     lc.numAttrs = 1;
-    if (b->march) {
+    if (march) {
         B_CK(cudaLaunchKernelEx(&lc, lbm::k_batch_march, (const lbm::BatchDomain*)b->d_doms, (const int4*)b->tasks.data,
                                 b->tasks.count, b->pool[0], b->pool[1], (const uint16_t*)b->d_flags,
                                 (const lbm_lattice_info*)b->d_info, b->d_macro, nsteps, b->cur, macro, b->d_bar,
@@ -589,7 +615,7 @@ int launch_persistent(lbm_batch* b, int nsteps, int skip_block, int skip_step, c
 
 int run_persistent_graph(lbm_batch* b, int nsteps) {
     int grid = 0;
-    B_TRY(persistent_grid(b, &grid));
+    B_TRY(persistent_grid(b, marches(b, nsteps), &grid));
     if (!b->graph || b->graph_steps != nsteps || b->graph_cur != b->cur || b->graph_grid != grid) {
         free_graph(b);
         cudaStream_t cs;
@@ -646,7 +672,7 @@ int run_steps(lbm_batch* b, int nsteps, int method) {
         b->launches += (uint64_t)nsteps * b->doms.size();
     }
     // a pass of fused steps swaps the pools once (their solid and padding cells hold zeros in both)
-    b->cur = (b->cur + (method == LBM_BATCH_PERSISTENT && b->march ? lbm::march_passes(nsteps) : nsteps)) & 1;
+    b->cur = (b->cur + (method == LBM_BATCH_PERSISTENT && marches(b, nsteps) ? lbm::march_passes(nsteps) : nsteps)) & 1;
     b->steps += nsteps;
     return LBM_OK;
 }
@@ -773,15 +799,13 @@ int lbm_batch_create(int32_t n, const lbm_domain_desc* desc, lbm_batch** out) {
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    size_t domain_cells = 0;
-    b->march = true;
-    for (const lbm::BatchDomain& dm : doms) {
-        b->march = b->march && dm.nx >= lbm::MARCH_W && dm.ny >= 8;
-        domain_cells += (size_t)dm.nx * dm.ny;
-    }
-    b->march = b->march && domain_cells >= BATCH_MARCH_CELLS;
+    b->can_march = live >= BATCH_MARCH_CELLS;
+    for (const lbm::BatchDomain& dm : doms) b->can_march = b->can_march && dm.nx >= lbm::MARCH_W && dm.ny >= 8;
     int r = e == cudaSuccess ? build_tiles(b) : bfail(LBM_ERR_CUDA, "batch set-up: %s", cudaGetErrorString(e));
-    if (r == LBM_OK && b->march) r = set_march_rows(b, march_rows_for(b));
+    if (r == LBM_OK && b->can_march) {
+        r = set_march_rows(b, march_rows_for(b));
+        b->march = r == LBM_OK && march_share(b, b->march_rows) >= MARCH_SHARE;
+    }
     if (r != LBM_OK) {
         lbm_batch_destroy(b);
         return r;
@@ -892,17 +916,18 @@ int lbm_batch_tune(lbm_batch* b, int32_t trial_steps, lbm_batch_config* best_out
     B_TRY(check_batch(b));
     if (trial_steps < 1) return bfail(LBM_ERR_ARG, "trial_steps must be >= 1");
     B_CK(cudaSetDevice(b->device));
-    const TuneKey key{(long)std::lround(std::log2((double)b->live_cells + 1.0) * 4.0), (int)b->doms.size(), b->device, b->march};
+    const TuneKey key{(long)std::lround(std::log2((double)b->live_cells + 1.0) * 4.0), (int)b->doms.size(), b->device,
+                      b->can_march ? 1 + (int)std::lround(32.0 * march_share(b, march_rows_for(b))) : 0};
     auto it = g_tune_cache.find(key);
     if (it != g_tune_cache.end()) {
         B_TRY(lbm_batch_set_config(b, &it->second.cfg));
-        if (b->march) B_TRY(set_march_rows(b, it->second.rows));
+        if (it->second.rows > 0) B_TRY(set_march_rows(b, it->second.rows));
+        b->march = it->second.rows > 0;
+        free_graph(b);
         if (best_out) *best_out = it->second.cfg;
         return LBM_OK;
     }
-    // the tile shapes first (they serve the other methods, and this one where k_batch_march cannot)
-    const bool march = b->march;
-    b->march = false;
+    // the tile shapes first (they serve the other methods and short calls, and this one where k_batch_march is slower)
     struct Restore {
         lbm_batch* b;
         bool march;
@@ -910,7 +935,8 @@ int lbm_batch_tune(lbm_batch* b, int32_t trial_steps, lbm_batch_config* best_out
             b->march = march;
             free_graph(b);
         }
-    } restore{b, march};
+    } restore{b, b->march};
+    b->march = false;
     free_graph(b);
     const int cpts[] = {0, 1, 4, 10, 11};  // 0: linear tiles; + 10: the 32-register budget
     const int txs[] = {32, 64, 128, 256};
@@ -938,7 +964,7 @@ int lbm_batch_tune(lbm_batch* b, int32_t trial_steps, lbm_batch_config* best_out
                 c.method = LBM_BATCH_PERSISTENT;
                 if (lbm_batch_set_config(b, &c) != LBM_OK) continue;
                 int grid = 0;
-                if (persistent_grid(b, &grid) != LBM_OK) continue;
+                if (persistent_grid(b, false, &grid) != LBM_OK) continue;
                 if (bp > 0 && grid != bp * b->sms) continue;  // over the occupancy limit: same as a smaller bp
                 if (run_steps(b, 2, LBM_BATCH_PERSISTENT) != LBM_OK) continue;  // warm-up (and graph capture)
                 B_CK(cudaEventRecord(e0, b->stream));
@@ -956,16 +982,15 @@ int lbm_batch_tune(lbm_batch* b, int32_t trial_steps, lbm_batch_config* best_out
                 }
             }
         }
-    int r = lbm_batch_set_config(b, &best);
-    if (march && r == LBM_OK) {
-        // the rows of a task, timed on single passes from the current pool into the other one, which
-        // leave the state where it is
+    int r = lbm_batch_set_config(b, &best), rows = 0;
+    if (b->can_march && r == LBM_OK) {
+        // the rows of a task, timed on single passes from the current pool into the other one, which leave the
+        // state where it is (and count a launch for three steps, so the march is kept where it wins on short calls, too)
         b->march = true;
-        best_ms = 1e30f;
-        int best_rows = b->march_rows;
-        for (int rows : {march_rows_for(b), 16, 24, 32, 48}) {
+        const int first = b->march_rows;
+        for (int trial : {march_rows_for(b), 16, 24, 32, 48}) {
             float ms = 0.0f;
-            if (r == LBM_OK) r = set_march_rows(b, rows);
+            if (r == LBM_OK) r = set_march_rows(b, trial);
             for (int i = 0; i < 4 && r == LBM_OK; ++i) {
                 if (i == 1) cudaEventRecord(e0, b->stream);
                 r = launch_persistent(b, 3, -1, -1, b->stream, false);
@@ -974,16 +999,17 @@ int lbm_batch_tune(lbm_batch* b, int32_t trial_steps, lbm_batch_config* best_out
             if (r == LBM_OK) r = read_status(b);
             if (r == LBM_OK && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess && ms / 9.0f < best_ms) {
                 best_ms = ms / 9.0f;
-                best_rows = rows;
+                rows = trial;
             }
         }
-        if (r == LBM_OK) r = set_march_rows(b, best_rows);
+        if (r == LBM_OK) r = set_march_rows(b, rows > 0 ? rows : first);
+        if (r == LBM_OK) restore.march = rows > 0;
         b->cfg.ms_per_step = best.ms_per_step = best_ms;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     B_TRY(r);
-    g_tune_cache[key] = {best, march ? b->march_rows : 0};
+    g_tune_cache[key] = {best, rows};
     if (best_out) *best_out = best;
     return LBM_OK;
 }

@@ -73,3 +73,37 @@ def test_fused_steps_have_a_grid_of_their_own(gpu):
     stream.synchronize()
     assert e[0].elapsed_time(e[1]) / 300 <= 1.5 * ms
     b.close()
+
+
+def _takes_fused_steps(batch, nsteps):
+    """Whether a call of nsteps does: the tile form of one block per SM has no block 2 x SMs, whose absence would be
+    noticed (the state is of no use afterwards)."""
+    import torch
+
+    from simuverse_gb300 import _native as nat
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    batch.configure(blocks_per_sm=1)
+    rc = batch.inject_missing_arrival(nsteps=nsteps, block=2 * sms, step=0, timeout_ns=200_000_000)
+    assert rc in (0, nat.LBM_ERR_TIMEOUT)
+    return rc != 0
+
+
+def _equal(n, nx, ny, scene):
+    return [dict(nx=nx, ny=ny, scene=scene, tau=0.7, speed=0.05)] * n
+
+
+@pytest.mark.parametrize("domains,pays", [
+    (_equal(1000, 64, 64, "channel"), False), (_equal(512, 64, 64, "channel"), False), (_equal(260, 64, 128, "cavity"), False), (_equal(64, 121, 300, "channel"), False),
+    (_equal(128, 181, 181, "cavity"), False), (_equal(128, 1024, 16, "channel"), False),
+    (_equal(40, 300, 200, "cavity"), True), (_equal(4, 1000, 700, "cavity"), True), ([BIG], True)])
+def test_where_fused_steps_pay(gpu, domains, pays):
+    b = BatchSimulator(domains)
+    assert _takes_fused_steps(b, 3) == pays
+    assert not _takes_fused_steps(b, 2)
+    b.close()
+    if len(domains) > 1:  # (the two forms tie on the one channel)
+        b = BatchSimulator(domains)
+        b.tune(trial_steps=10)
+        assert _takes_fused_steps(b, 3) == pays
+        b.close()

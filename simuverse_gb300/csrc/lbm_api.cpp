@@ -427,6 +427,7 @@ int scene_and_state_on_device(lbm_handle* h) {
     }
     h->host_info.clear();
     h->host_info_lazy = true;
+    h->rows = lbm::scene_rows(h);
     h->no_solids = h->p.scene == LBM_SCENE_PERIODIC;
     h->faces = h->p.scene == LBM_SCENE_CHANNEL;  // the inlet in the first column, the outflow in the last one
     h->outlets_last = true;
@@ -477,6 +478,13 @@ void restart_countdown(lbm_handle* h, int y0, int y1) {
     const lbm_lattice_info* rows = h->host_info.data() + (size_t)y0 * h->nx;
     h->countdown = std::max(h->countdown, longest_countdown(rows, (size_t)(y1 - y0) * h->nx));
 }
+// h->rows of records that the host wrote, from their flags (asynchronous: the caller waits for the stream)
+int count_rows(lbm_handle* h) {
+    if (!lbm::has_fused_form(h)) return LBM_OK;
+    LBM_CK(lbm::launch_count_rows(h, h->stream));
+    LBM_CK(cudaMemcpyAsync(&h->rows, h->d_count + 1, sizeof(h->rows), cudaMemcpyDeviceToHost, h->stream));
+    return LBM_OK;
+}
 // The same over the device's records, which were all replaced, and whether the walls' slots that no step writes
 // hold the same in both buffers (a new solid cell keeps what it held as fluid, another step in each; new
 // velocities change nothing).  Waits for the stream.
@@ -484,7 +492,8 @@ int recount(lbm_handle* h) {
     unsigned long long n = 0, differ = 1;
     LBM_CK(lbm::launch_longest_countdown(h, h->stream));
     LBM_CK(cudaMemcpyAsync(&n, h->d_count, sizeof(n), cudaMemcpyDeviceToHost, h->stream));
-    if (h->p.dtype == LBM_DTYPE_F32 && h->p.kernel == LBM_KERNEL_AUTO) {  // the others take single steps
+    LBM_TRY(count_rows(h));
+    if (lbm::has_fused_form(h)) {  // the others take single steps
         LBM_CK(lbm::launch_count_solid_slots(h, h->stream));
         LBM_CK(cudaMemcpyAsync(&differ, h->d_count, sizeof(differ), cudaMemcpyDeviceToHost, h->stream));
     }
@@ -697,7 +706,7 @@ int lbm_create(const lbm_params* pin, lbm_handle** out) {
     if (e == cudaSuccess) e = pool_alloc(&h->d_info, h->N * sizeof(lbm_lattice_info), s);
     if (e == cudaSuccess) e = pool_alloc(&h->d_macro, 3 * h->N * sizeof(float), s);
     if (e == cudaSuccess) e = pool_alloc(&h->d_part, (size_t)lbm::RED_BLOCKS * 6 * sizeof(double) + 64 * sizeof(double), s);
-    if (e == cudaSuccess) e = pool_alloc(&h->d_count, sizeof(unsigned long long), s);
+    if (e == cudaSuccess) e = pool_alloc(&h->d_count, 6 * sizeof(unsigned long long), s);
     if (e == cudaSuccess) e = pool_alloc(&h->d_status, sizeof(int), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(h->d_status, 0, sizeof(int), s);
     if (e != cudaSuccess) {
@@ -715,6 +724,7 @@ int lbm_create(const lbm_params* pin, lbm_handle** out) {
         if (r == LBM_OK) r = init_state(h);
     }
     if (r == LBM_OK) r = rebuild_flags(h);
+    if (r == LBM_OK && !device_scene(p)) r = count_rows(h);
     const int rs = sync(h);                  // also after a failed launch: the copy reads the list
     h->scene_disks = std::vector<double>();
     if (r == LBM_OK) r = rs;
@@ -809,6 +819,7 @@ int lbm_reset(lbm_handle* h) {
         if (r == LBM_OK) r = init_state(h);
     }
     if (r == LBM_OK) r = rebuild_flags(h);
+    if (r == LBM_OK && !device_scene(h->p)) r = count_rows(h);
     // no record counts down: a new scene has permanent ones only, and init.wgsl ends the others
     if (r == LBM_OK) h->countdown = 0;
     h->pre_x = h->pre_y = 0.0f;  // fluid_simulator.rs:214

@@ -29,6 +29,15 @@ struct LbmRange {
 };
 #endif
 
+namespace lbm {
+// Rows of windows of 60 columns and two more on each side, by what some cell of theirs is (h->rows): a forcing cell; that
+// or one beside a moving wall; an inlet or outflow (reference mode: a forcing cell, or one on the outer ring beside a
+// wall); anything but plain fluid; a wall inside, two cells or more from the border
+struct RowCounts {
+    unsigned long long forced = 0, rare = 0, face = 0, mixed = 0, inner = 0;
+};
+}  // namespace lbm
+
 struct lbm_handle {
     lbm_params p;
     int nx = 0, ny = 0;
@@ -66,6 +75,8 @@ struct lbm_handle {
     // and what those of small lattices ask (lbm_step_cluster.cu): no outflow cell outside the last column; any
     // inlet or outflow cell
     bool outlets_last = true, faces = false;
+    // and what both ask: how many rows of the march's windows (lbm_march.cuh) hold a cell whose step takes longer
+    lbm::RowCounts rows;
     bool stepped_since_init = false;  // macro_tex holds (0,0,0,1) right after init
     float pre_x = 0.0f, pre_y = 0.0f;  // FluidSimulator::pre_pos
     int device = 0;
@@ -165,6 +176,12 @@ inline void took_steps(lbm_handle* h, int n, bool cluster) {
     h->behind_cluster = cluster;
     h->behind_omega = h->omega;
 }
+// The lattice's kernels have a form that takes several steps per launch.
+bool has_fused_form(const lbm_handle* h);
+// counts h->rows from the flags into d_count[1 ..] (asynchronous), or says what they are for a scene of physics mode that is
+// built on the device
+cudaError_t launch_count_rows(lbm_handle* h, cudaStream_t s);
+RowCounts scene_rows(const lbm_handle* h);
 // fused steps (lbm_step_fused.cu): how many of the next `left` steps one launch takes (1: launch_step)
 int fused_steps(const lbm_handle* h, int left);
 cudaError_t launch_fused(lbm_handle* h, int steps, bool write_macro, cudaStream_t s);

@@ -9,8 +9,8 @@ from test_gpu_fused import _same
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nx,ny,scene,form,n", [(1100, 800, "cavity", dict(mode="physics"), 2), (1100, 800, "channel", dict(mode="physics", collision="kbc"), 8),
-                                                (1100, 800, "poiseuille", dict(mode="reference", arith="fast"), 2),
+@pytest.mark.parametrize("nx,ny,scene,form,n", [(1300, 1250, "cavity", dict(mode="physics"), 2), (1300, 1250, "channel", dict(mode="physics", collision="kbc"), 8),
+                                                (1700, 1650, "poiseuille", dict(mode="reference", arith="fast"), 2),
                                                 (128, 128, "channel", dict(mode="physics"), 16)])
 def test_captured_steps(gpu, nx, ny, scene, form, n):
     import torch

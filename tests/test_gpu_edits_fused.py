@@ -13,9 +13,10 @@ from test_gpu_fused import ROOT, _same
 
 pytestmark = pytest.mark.gpu
 
-# lattices of fused steps (march) and, in physics mode, of one cluster
-LARGE, SMALL = (1100, 800), (128, 128)
-FORMS = [(LARGE, "poiseuille", dict(mode="reference", arith="fast")), (LARGE, "custom", dict(mode="reference", arith="fast"))]
+# lattices of fused steps (march), of two of them as well, and, in physics mode, of one cluster
+LARGE, SMALL = (1300, 1250), (128, 128)
+FORMS = [((1700, 1650), "poiseuille", dict(mode="reference", arith="fast")),
+         ((1500, 1350), "custom", dict(mode="reference", arith="fast"))]
 FORMS += [(size, scene, dict(mode="physics", collision=c)) for size in (LARGE, SMALL)
           for scene, c in (("channel", "bgk"), ("periodic", "bgk"), ("cavity", "kbc"))]
 IDS = ["%s %s %s" % (s[0], sc, f.get("collision", "reference")) for s, sc, f in FORMS]
@@ -54,10 +55,11 @@ def _fused(pair, n):
 @pytest.mark.parametrize("n", [2, 3, 4, 7, 16, 17])
 def test_edits_between_calls(gpu, size, scene, form, n):
     nx, ny = size
+    if size != SMALL and n > 7:
+        pytest.skip("the last launch is one of 2 or 3 steps")
     pair = _pair(size, scene, form)
     fused = _fused(pair, n)
-    # other shapes of call: small lattices take some ten steps a launch
-    assert fused or size == SMALL and n < 16
+    assert fused or size == SMALL and n < 16  # (small lattices take ten steps or so a launch)
     x, y = 29, ny // 2  # reaches columns 1 and 0
     _both(pair, lambda s: s.add_obstacle(x, y))
     _both(pair, lambda s: s.step(5))
@@ -115,11 +117,11 @@ def test_what_else_keeps_the_other_buffer(gpu, tmp_path, size, scene, form, n):
         _same(*pair, "reset")
 
 
-@pytest.mark.parametrize("scene,form", [("custom", dict(mode="reference", arith="fast")), ("cavity", dict(mode="physics"))])
-def test_unlike_walls_do_not_outlive_their_cause(gpu, tmp_path, scene, form):
+@pytest.mark.parametrize("size,scene,form", [FORMS[1], (LARGE, "cavity", dict(mode="physics"))], ids=["reference", "physics"])
+def test_unlike_walls_do_not_outlive_their_cause(gpu, tmp_path, size, scene, form):
     """New records that leave the walls as they were, and a checkpoint of a lattice whose walls agree: a frame of two
     steps is one launch."""
-    a, b = _pair(LARGE, scene, form)
+    a, b = _pair(size, scene, form)
     _both((a, b), lambda s: s.step(3))
     info = a.info()
     info["vx"][5, 5] = 0.01
@@ -130,7 +132,7 @@ def test_unlike_walls_do_not_outlive_their_cause(gpu, tmp_path, scene, form):
     _same(a, b, "records")
     path = str(tmp_path / "walls")
     b.save(path)
-    c = _pair(LARGE, scene, form)[0]
+    c = _pair(size, scene, form)[0]
     c.load(path)
     before = c.kernel_launches
     _both((c, b), lambda s: s.compute())
@@ -146,7 +148,7 @@ def child_main():
     lib = nat.load()
     assert nat.LIB_PATH.endswith("liblbm_bounds.so")
     for size, scene, form in FORMS:
-        for n in (2, 3, 16):
+        for n in (16,) if size == SMALL else (2, 3):
             test_edits_between_calls(lib, size, scene, form, n)
     n = ctypes.c_uint64()
     assert lib.lbm_bounds_report(ctypes.byref(n), None, None, None) == 0 and n.value == 0

@@ -397,8 +397,7 @@ static cudaError_t cluster_ready(int device, int* ready) {
 }
 
 int cluster_steps(const lbm_handle* h, int left) {
-    if (left < 4 || h->p.mode != LBM_MODE_PHYSICS || h->p.dtype != LBM_DTYPE_F32 ||
-        h->p.kernel != LBM_KERNEL_AUTO || !core_has(h->p.collision) || h->p.macro_every_step || h->countdown > 0 ||
+    if (left < 4 || h->p.mode != LBM_MODE_PHYSICS || !has_fused_form(h) || h->p.macro_every_step || h->countdown > 0 ||
         !h->outlets_last || h->ny < CL_BLOCKS || h->nx > CL_COLUMNS || cluster_rows(h) > CL_ROWS ||
         cluster_rows(h) * h->nx > CL_CELLS)
         return 1;
@@ -408,16 +407,25 @@ int cluster_steps(const lbm_handle* h, int left) {
     // (four) 1.4 and 2.0 in a periodic box and 1.4 and 1.5 in a cavity; calls of 4 steps lose there (0.8 and
     // 1.0), and 300^2 (seven rows) lost up to a third alone.  Inlets and outflows, and KBC, take longer a row:
     // 192^2 gains 1.0 to 1.2 alone and 1.4 to 1.8 in calls of 16 and 64 steps, 256^2 ran 0.8 alone.
-    const int sets = cluster_sets(h->nx), warp_rows = (cluster_rows(h) + sets - 1) / sets;
-    const bool costly = h->faces || h->p.collision == LBM_COLLISION_KBC;
+    const int windows = cluster_windows(h->nx), sets = cluster_sets(h->nx), warp_rows = (cluster_rows(h) + sets - 1) / sets;
+    const bool kbc = h->p.collision == LBM_COLLISION_KBC, costly = h->faces || kbc;
     if (warp_rows > (costly ? 3 : 4) || left < (costly ? (warp_rows < 3 ? 6 : 16) : 2 * warp_rows + 2)) return 1;
+    // A step ends with its slowest warp.  Forcing cells run a function of their own, in memory, for the whole row: with
+    // 1 % of them BGK ran 0.87 to 1.4 times as fast as single steps at 128^2, 0.6 to 0.9 at 192^2, 0.44 to 0.6 at 256^2
+    // (all of them 0.75, 0.45 and 0.32), KBC 0.7 to 1.2, 0.5 and so down; only BGK on 64^2, with four rows to a block,
+    // gains (1.0 to 1.9).  Moving walls through the lattice: 1.4 to 2.8 to 128^2, KBC at 192^2 0.8.  Four rows to a warp
+    // gain while plain ones are among them (a cavity's walls: 40 % of the rows): with walls everywhere 0.7 to 0.96.
+    const RowCounts& n = h->rows;
+    if (n.forced > 16 && (kbc || cluster_rows(h) * windows > 4)) return 1;
+    if (kbc && warp_rows >= 3 && n.rare > 2ull * windows + 48) return 1;
+    if (warp_rows >= 4 && 10 * n.mixed > 6ull * windows * (unsigned)h->ny) return 1;
     int ready = 0;
     const cudaError_t e = h->p.collision == LBM_COLLISION_KBC ? cluster_ready<LBM_COLLISION_KBC>(h->device, &ready)
                                                               : cluster_ready<LBM_COLLISION_BGK>(h->device, &ready);
     if (e != cudaSuccess) cudaGetLastError();  // not for the next launch's check
     if (e != cudaSuccess || ready < 1) return 1;
-    const int n = std::min(left, CL_MOST_STEPS);
-    return n % 2 == 1 || even_steps(h) ? n : n - 1;
+    const int steps = std::min(left, CL_MOST_STEPS);
+    return steps % 2 == 1 || even_steps(h) ? steps : steps - 1;
 }
 
 template <int COLL>

@@ -1,4 +1,4 @@
-"""Where steps are fused: launches of a call on both sides of each line of the rules (march_pays), and the
+"""Where steps are fused: launches of a call on both sides of each line of the rules (march_pays, cluster_steps), and the
 state of single steps on either."""
 import numpy as np
 import pytest
@@ -40,7 +40,11 @@ KBC = dict(collision="kbc")
     (1032, 780, "channel", {}, None, 3, 3), (64, 12504, "channel", {}, None, 3, 3), (1032, 780, "channel", {}, "solid", 3, 1), (1000, 1000, "channel", KBC, "solid", 3, 1),
     (301, 2700, "custom", REF, None, 2, 2),
     (1500, 1500, "periodic", {}, "column", 3, 3), (3000, 3000, "periodic", {}, "column", 3, 1), (1500, 1500, "periodic", {}, "force", 3, 3),
-    (1500, 1500, "periodic", KBC, "moving", 2, 2), (1500, 1500, "periodic", {}, "solid", 3, 1)])
+    (1500, 1500, "periodic", KBC, "moving", 2, 2), (1500, 1500, "periodic", {}, "solid", 3, 1),
+    # small lattices
+    (128, 128, "periodic", {}, None, 20, 1), (128, 128, "periodic", {}, "force", 20, 20), (64, 64, "periodic", {}, "force", 20, 1),
+    (64, 64, "periodic", KBC, "force", 20, 20), (192, 192, "periodic", KBC, "moving", 20, 20),
+    (192, 192, "periodic", {}, "moving", 20, 1), (256, 256, "periodic", {}, "solid", 20, 20), (256, 256, "periodic", {}, None, 20, 1)])
 def test_launches(gpu, nx, ny, scene, form, kind, steps, launches):
     from simuverse_gb300 import FluidSimulator
 

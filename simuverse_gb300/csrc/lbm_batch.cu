@@ -184,21 +184,20 @@ __global__ void __launch_bounds__(256, batch_min_blocks(KF)) k_batch_persistent(
         if (!grid_barrier(bar, (unsigned)(s + 1) * gridDim.x, timeout_ns, s)) return;
     }
 }
-// method 0 for batches whose domains are wide and tall enough: passes of up to three fused steps
-// (lbm_march.cuh).  A warp takes windows of 60 columns x some rows of a domain from a common counter,
+// method 0 for calls of three steps or more of batches whose domains fill its windows (march_share): passes of three
+// fused steps, or two (lbm_march.cuh).  A warp takes windows of 60 columns x some rows of a domain from a common counter,
 // since those at walls, inlets and outflows take longer (124 and 91 GLUPS where every window is one of
 // them, 180 inside); the blocks meet at the grid barrier once per pass.  One step per pass moves 74 bytes
 // per cell and ran at 86 % of the measured copy bandwidth; three move about 26.  256 domains of 64 to
 // 1024 cells a side: 80 -> 117 GLUPS, 64 domains 77 -> 89 (what bounds those: two to three tasks per
 // warp and pass, uneven ones, and windows that a domain's width fills badly).
-// the last pass of a call that is no multiple of three steps: a function, which costs the loop nothing
-template <int T>
-__device__ __noinline__ void march_rest(const FusedLattice& L, const BgkConst<float2>& k, int x0, int y0, int y1, bool macro,
+// a pass of two steps, in calls that are no multiple of three: a function, which costs the loop nothing
+__device__ __noinline__ void march_two(const FusedLattice& L, const BgkConst<float2>& k, int x0, int y0, int y1, bool macro,
                                         uint32_t smem) {
-    march_window<T, LBM_COLLISION_BGK, true>(L, k, x0, y0, y1, macro, smem);
+    march_window<2, LBM_COLLISION_BGK, true>(L, k, x0, y0, y1, macro, smem);
 }
 constexpr int BM_WARPS = 4;   // warps of a block, each on its own
-constexpr int BM_BLOCKS = 3;  // blocks per SM the kernel is compiled for: 168 registers, no spills
+constexpr int BM_BLOCKS = 3;  // blocks per SM the kernel is compiled for: 168 registers, 40 bytes of spills
 __global__ void __launch_bounds__(32 * BM_WARPS, BM_BLOCKS)
     k_batch_march(const BatchDomain* __restrict__ doms, const int4* __restrict__ tasks, int ntasks, float* pool0,
                   float* pool1, const uint16_t* flags, const lbm_lattice_info* info, float* macro, int nsteps, int cur0,
@@ -209,7 +208,7 @@ __global__ void __launch_bounds__(32 * BM_WARPS, BM_BLOCKS)
     const uint32_t smem = (uint32_t)__cvta_generic_to_shared(march_mem) + (uint32_t)(wid * march_smem(3));
     const int warps = (int)gridDim.x * BM_WARPS;
     for (int done = 0, pass = 0; done < nsteps; ++pass) {
-        const int left = nsteps - done, T = left == 4 ? 2 : min(left, 3);
+        const int left = nsteps - done, T = left == 4 ? 2 : min(left, 3);  // never 1: calls have two steps or more
         const bool odd = ((cur0 + pass) & 1) != 0, mac = write_macro && left == T;
         if (blockIdx.x == 0 && threadIdx.x == 0) bar->ticket[(pass + 1) % 3] = 0;  // the next pass's, last used two passes ago
         int t = (int)blockIdx.x * BM_WARPS + wid;
@@ -235,8 +234,7 @@ __global__ void __launch_bounds__(32 * BM_WARPS, BM_BLOCKS)
             __syncwarp();
             const BgkConst<float2> k(dm.omega);
             if (T == 3) march_window<3, LBM_COLLISION_BGK, true>(L, k, q.y, q.z, q.w, mac, smem);
-            else if (T == 2) march_rest<2>(L, k, q.y, q.z, q.w, mac, smem);
-            else march_rest<1>(L, k, q.y, q.z, q.w, mac, smem);
+            else march_two(L, k, q.y, q.z, q.w, mac, smem);
             t = warps + (int)__shfl_sync(0xffffffffu, next, 0);
         }
         if ((int)blockIdx.x == skip_block && skip_step >= done && skip_step < done + T) return;  // injected (tests)

@@ -479,7 +479,7 @@ struct DwLayout {
     static constexpr int OFF_ONES = 3 * XC * PLANE_B;   // a plane of ones, after the input's [row][group]
     static constexpr int OFF_G = OFF_ONES + PLANE_B;    // gradient planes
     static constexpr int STAGE = (3 * XC + 1 + GC > 16 ? 3 * XC + 1 + GC : 16) * PLANE_B;  // (M = 128 reads sixteen)
-        static constexpr int NSTAGE = 4;                    // (six or eight measured 1 to 4 % slower)
+    static constexpr int NSTAGE = 4;                    // (six or eight measured 1 to 4 % slower)
     static constexpr int OFF_BAR = NSTAGE * STAGE;      // full[NSTAGE], empty[NSTAGE], done
     static constexpr int OFF_TSLOT = OFF_BAR + 8 * (2 * NSTAGE + 1);
     static constexpr int SMEM = OFF_TSLOT + 8;

@@ -68,7 +68,7 @@ constexpr int SLOT_FLAGS = 9 * MARCH_RAW * 4;  // byte offset of the flag words
 constexpr int SLOT_BYTES = SLOT_FLAGS + ((MARCH_RAW * 2 + 15) / 16) * 16;
 constexpr int KEPT_OFF = 5 * SLOT_BYTES;            // own outgoing populations 1 .. 8 of steps 1 and 2
 // bytes per warp that fuses t steps
-__host__ __device__ constexpr int march_smem(int t) { return KEPT_OFF + (t > 1 ? t - 1 : 0) * 8 * 256; }
+__host__ __device__ constexpr int march_smem(int t) { return KEPT_OFF + (t - 1) * 8 * 256; }
 
 // The copies of a warp.  VEC (rows a multiple of 4 cells long): 16-byte copies of four cells, two
 // planes at a time by the two halves of the warp, then the seventeenth chunk of all nine planes;
@@ -235,7 +235,7 @@ __device__ __forceinline__ void march_row(float2 (&d)[9], uint32_t own, int stri
 template <int T, int COLL, bool VEC>
 __device__ __forceinline__ void march_window(const FusedLattice& L, const BgkConst<float2>& kin, int x0, int y0, int y1,
                                              bool macro, uint32_t smem) {
-    static_assert(T >= 1 && T <= 3, "steps of one pass");
+    static_assert(T == 2 || T == 3, "steps of one pass");
     constexpr int HALO = T - 1;
     constexpr int IN = 4 - HALO;  // the window's first column in a slot
     int lane = threadIdx.x & 31;
@@ -289,7 +289,7 @@ __device__ __forceinline__ void march_window(const FusedLattice& L, const BgkCon
         const InletVel v0 = vn;
         fn = flags_of(sp, yl);
         vn = inlet_vel(fn, xa, xb, yl, L);
-        const int ys = T == 1 ? yr : (T == 2 ? ym : (ym == 0 ? L.ny - 1 : ym - 1));  // row of step T
+        const int ys = T == 2 ? ym : (ym == 0 ? L.ny - 1 : ym - 1);  // row of step T
 
         const auto rows = [&](auto mixed) {
             constexpr bool MIXED = decltype(mixed)::value;
@@ -299,7 +299,7 @@ __device__ __forceinline__ void march_window(const FusedLattice& L, const BgkCon
             };
             float2 d1[9], d2[9], d3[9], C1[9], C2[9], o[9], rho, nux, nuy;
             // pulls from the rings first: their registers take the new rows
-            if (T > 1) ring_pulls<MIXED>(R1, lane, c1, f1, c0, f0, d2);
+            ring_pulls<MIXED>(R1, lane, c1, f1, c0, f0, d2);
             if (T > 2) ring_pulls<MIXED>(R2, lane, c2, f2, c1, f1, d3);
 #pragma unroll
             for (int j = 0; j < 9; ++j)
@@ -310,22 +310,15 @@ __device__ __forceinline__ void march_window(const FusedLattice& L, const BgkCon
                 if ((f0 & FL_MAT_MASK) == LBM_OUTLET) { d1[3].x = e3.x; d1[6].x = e6.x; d1[7].x = e7.x; }
                 if (((f0 >> 16) & FL_MAT_MASK) == LBM_OUTLET) { d1[3].y = e3.y; d1[6].y = e6.y; d1[7].y = e7.y; }
             }
-            march_row<COLL, MIXED>(d1, s0 + 4 * MARCH_RAW, 4 * MARCH_RAW, c0, f0, v0, xa, xb, yr, L, k,
-                                   T == 1 ? o : C1, rho, nux, nuy);
-            if constexpr (T > 1) {
-                ring_push<MIXED>(R1, C1, lane, c1, f1, d2);
-                march_row<COLL, MIXED>(d2, kept, 256, c1, f1, vel_of(c1, f1, ym), xa, xb, ym, L, k, T == 2 ? o : C2, rho,
-                                       nux, nuy);
-                if (MIXED && c0 != ROW_PLAIN) {
-                    keep_own(kept, c0, C1);
-                }
-            }
+            march_row<COLL, MIXED>(d1, s0 + 4 * MARCH_RAW, 4 * MARCH_RAW, c0, f0, v0, xa, xb, yr, L, k, C1, rho, nux, nuy);
+            ring_push<MIXED>(R1, C1, lane, c1, f1, d2);
+            march_row<COLL, MIXED>(d2, kept, 256, c1, f1, vel_of(c1, f1, ym), xa, xb, ym, L, k, T == 2 ? o : C2, rho, nux,
+                                   nuy);
+            if (MIXED && c0 != ROW_PLAIN) keep_own(kept, c0, C1);
             if constexpr (T > 2) {
                 ring_push<MIXED>(R2, C2, lane, c2, f2, d3);
                 march_row<COLL, MIXED>(d3, kept + 2048, 256, c2, f2, vel_of(c2, f2, ys), xa, xb, ys, L, k, o, rho, nux, nuy);
-                if (MIXED && c1 != ROW_PLAIN) {
-                    keep_own(kept + 2048, c1, C2);
-                }
+                if (MIXED && c1 != ROW_PLAIN) keep_own(kept + 2048, c1, C2);
             }
             if (r >= y0 + HALO) {
                 RowOut t;
@@ -334,12 +327,12 @@ __device__ __forceinline__ void march_window(const FusedLattice& L, const BgkCon
                 const int xe = min(x0 + MARCH_OUT, L.nx);
                 t.sa = t.ca >= x0 && t.ca < xe;
                 t.sb = t.ca + 32 >= x0 && t.ca + 32 < xe;
-                const unsigned fs = T == 1 ? f0 : (T == 2 ? f1 : f2);
+                const unsigned fs = T == 2 ? f1 : f2;
                 store_row(L, t, !MIXED || !is_solid((int)(fs & FL_MAT_MASK)),
                           !MIXED || !is_solid((int)((fs >> 16) & FL_MAT_MASK)), macro, o, rho, nux, nuy);
             }
         };
-        if ((c0 | (T > 1 ? c1 : 0) | (T > 2 ? c2 : 0)) == ROW_PLAIN) rows(std::false_type{});
+        if ((c0 | c1 | (T > 2 ? c2 : 0)) == ROW_PLAIN) rows(std::false_type{});
         else rows(std::true_type{});
 
         f2 = f1;

@@ -12,7 +12,8 @@ steps (repeated until about --min-seconds of device time, so that the clock samp
 load; `spread` gives the slowest and fastest interval); e2e = the same metric for the whole
 job through the public API (create from host parameters, scene mask built on the device
 from the uploaded disk list, K steps, macro field read back to page-locked host memory);
-roofline = 72 algorithmic bytes per cell update over the measured HBM copy bandwidth;
+roofline = 72 algorithmic bytes per cell and launch (per_step_frac: and step) over the measured
+HBM copy bandwidth;
 cpu_baseline = the oracle (the CPU restatement of the reference path) on the host cores,
 full workload, about 15 s of steps.  `reference_mode_glups` / `reference_mode_exact_glups`:
 the reference's own rules (its Poiseuille scene) at the same size, in the fast and the exact
@@ -256,10 +257,12 @@ def measure_sim(sim, stream, cells, bytes_per_cell, peak, steps=100, warmup=5, m
     sim.set_stream(stream.cuda_stream)
     sim.step(warmup)
     torch.cuda.synchronize()
+    launches0 = sim.kernel_launches
     ms = timed_intervals(sim.step, stream, steps, min_seconds, min_repeats=3)
+    fused = steps * (len(ms) + 1) / max(1, sim.kernel_launches - launches0)  # steps that share a launch's bytes
     g = glups_of(cells, steps, median(ms))
-    return {"glups": g, "gb_per_s": g * bytes_per_cell, "roofline_frac": g * bytes_per_cell / peak,
-            "bytes_per_cell": bytes_per_cell, "steps_per_interval": steps, "intervals": len(ms),
+    return {"glups": g, "gb_per_s": g * bytes_per_cell / fused, "roofline_frac": g * bytes_per_cell / fused / peak,
+            "steps_per_launch": fused, "per_step_frac": g * bytes_per_cell / peak, "bytes_per_cell": bytes_per_cell, "steps_per_interval": steps, "intervals": len(ms),
             "spread_glups": [glups_of(cells, steps, max(ms)), glups_of(cells, steps, min(ms))]}
 
 
@@ -305,7 +308,8 @@ def run_extras(args, stream, peak):
         ms = timed_intervals(b.step, stream, steps, 0.3, min_repeats=3)
         b.status()
         g = glups_of(b.cells, steps, median(ms))
-        res[method] = {"glups": g, "gb_per_s": 72 * g, "roofline_frac": 72 * g / peak, "steps_per_interval": steps,
+        # (how many steps a persistent launch fuses is not its caller's to see)
+        res[method] = {"glups": g, "per_step_frac": 72 * g / peak, "steps_per_interval": steps,
                        "intervals": len(ms)}
     res["persistent_over_loop"] = res["persistent"]["glups"] / res["domain_loop"]["glups"]
     b.close()
@@ -405,12 +409,12 @@ def run_gpu(args):
     ms = median(ms_list)
     ms_max = max_over_ranks(pg, ms, "cuda")
     value = replica_glups(world, cells, args.steps, ms_max * 1e-3)
-    per_launch_s = ms * 1e-3 / args.steps
+    per_step_s = ms * 1e-3 / args.steps
     bytes_per_cell = 18 * BYTES_PER_VALUE[args.dtype]
-    achieved = bytes_per_cell * cells / per_launch_s / 1e9
     peak, peak_kind = measured_peak()
-    # AUTO fuses FP32 steps: a launch moves a step's bytes for several of them
-    steps_per_launch = args.steps * len(ms_list) / max(1, gpu_launches)
+    # AUTO fuses FP32 steps: a launch moves a step's bytes for several of them (one interval more estimates the repeats)
+    steps_per_launch = args.steps * (len(ms_list) + 1) / max(1, gpu_launches)
+    achieved = bytes_per_cell * cells / (per_step_s * steps_per_launch) / 1e9
     tr = committed_traffic(args) if steps_per_launch <= 1.0 else None
 
     # ---- macro every step (the reference's behaviour), reported separately
@@ -477,8 +481,9 @@ def run_gpu(args):
                          "traffic_source": (tr or {}).get("source"),
                          "algorithmic_bytes_per_launch": bytes_per_cell * cells,
                          "steps_per_launch": steps_per_launch,
-                         "what": "achieved counts every step's populations once read and once written; "
-                                 "fused steps move them once per launch, so frac may exceed 1"},
+                         "per_step_frac": bytes_per_cell * cells / per_step_s / 1e9 / peak,
+                         "what": "achieved counts the populations once read and once written per launch, which fused "
+                                 "steps share; per_step_frac counts them for every step (1 bounds single steps)"},
             "macro_every_step_glups": glups_macro,
             "reference_mode_glups": glups_ref_mode.get("fast"),
             "reference_mode_exact_glups": glups_ref_mode.get("exact"),

@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
     // (< POS), loaded ahead of their use: the second warpgroup has the first 128 positions, as the first
     // one writes the projected outputs (with both on the first, and a wait for each layer's accumulators, a
     // call on 1024^2 took 89.7 us; now 88.2.  What bounds it: a step's MMAs and its epilogues take turns,
-    // the tensor pipe is busy for 41 % with two blocks on the SM)
+    // the tensor pipe is busy for 41 % (sm__pipe_tc_cycles_active) with two blocks on the SM)
     static_assert(POS <= TC_THREADS, "one position a thread");
     const int fp = (tid + TC_THREADS / 2) % TC_THREADS;
     float pre[9];

@@ -536,8 +536,8 @@ struct Scratch {
 // the state one step before the current one.  It is called before anything that makes the other buffer's content
 // last: a cell that turns solid keeps it (ring cells of the reference's rules pull from it, and it is there
 // when the cell turns fluid again), checkpoints hold both buffers, and an initialisation leaves fluid cells of one
-// as they are.  A launch of several steps computes with records and flags that do not change, so its
-// steps can be taken again.  Asynchronous on the handle's stream.
+// as they are; and before every change of a record.  A launch of several steps computes with records and flags
+// that do not change, so with the same ones its steps can be taken again.  Asynchronous on the handle's stream.
 int catch_up(lbm_handle* h) {
     if (h->behind < 2) return LBM_OK;
     const int n = h->behind - 1, cur = h->cur;
@@ -902,6 +902,7 @@ int lbm_add_external_force(lbm_handle* h, float pos_x, float pos_y, float pre_x,
     if (h->p.pixel_size < 2)
         return fail(LBM_ERR_ARG, "force strokes need pixel_size >= 2 (the reference divides by pixel_size - 1)");
     LBM_TRY(use_device(h));
+    LBM_TRY(catch_up(h));  // with the records and flags of those steps
     h->countdown = std::max<int64_t>(h->countdown, FORCE_STEPS);
     std::vector<size_t> cells;
     const lbm_lattice_info rec = force_stroke(h->nx, h->ny, h->p.pixel_size, pos_x, pos_y, pre_x, pre_y, cells);
@@ -980,7 +981,7 @@ int lbm_apply_edits(lbm_handle* h, const lbm_edit* edits, int32_t n, int32_t* ap
         }
     }
     LBM_TRY(use_device(h));
-    if (!obs.empty()) LBM_TRY(catch_up(h));
+    if (!obs.empty() || !forces.empty()) LBM_TRY(catch_up(h));
     // a cell written by several strokes keeps the last one
     if (forces.size() > 1) {
         std::vector<size_t> order(forces.size());

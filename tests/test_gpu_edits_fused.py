@@ -118,6 +118,28 @@ def test_what_else_keeps_the_other_buffer(gpu, tmp_path, size, scene, form, n):
         _same(*pair, "reset")
 
 
+@pytest.mark.parametrize("size,scene,form", FORMS, ids=IDS)
+@pytest.mark.parametrize("stroke", ["call", "list"])
+def test_records_that_change_before_the_walls(gpu, tmp_path, size, scene, form, stroke):
+    """A stroke, then an obstacle or a checkpoint, without a step between: its records have counted nothing yet, and what is
+    made up for was computed without them."""
+    nx, ny = size
+    pair = _pair(size, scene, form)
+    line = (nx + 90.0, ny + 40.0, nx - 90.0, ny - 40.0)
+    force = (lambda s: s.add_external_force(line[:2], line[2:])) if stroke == "call" else (lambda s: s.apply_edits([("force",) + line]))
+    assert _fused(pair, 19)
+    _both(pair, force)
+    for k, s in enumerate(pair):
+        s.save(str(tmp_path / ("%d" % k)))
+    with open(tmp_path / "0", "rb") as a, open(tmp_path / "1", "rb") as b:
+        assert a.read() == b.read()
+    _both(pair, lambda s: s.add_obstacle(nx // 2 + 20, ny // 2))
+    assert np.array_equal(pair[0].info(), pair[1].info())
+    for k in (1, 4):
+        _both(pair, lambda s: s.step(k))
+        _same(*pair, "obstacle")
+
+
 @pytest.mark.parametrize("size,scene,form", [FORMS[1], (LARGE, "cavity", dict(mode="physics"))], ids=["reference", "physics"])
 def test_unlike_walls_do_not_outlive_their_cause(gpu, tmp_path, size, scene, form):
     """New records that leave the walls as they were, and a checkpoint of a lattice whose walls agree: a frame of two

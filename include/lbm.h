@@ -74,8 +74,8 @@ extern "C" {
 
 /* step kernel variants (physics mode) */
 #define LBM_KERNEL_AUTO 0   /* the fastest measured variant: LBM_KERNEL_CELL for FP32 / FP64 (FP32 BGK
-                               and KBC lattices of about a million cells or more take up to three steps
-                               per launch, by their size, width, walls and forcing cells; small ones, to
+                               and KBC lattices of 800,000 cells or more take up to three steps per
+                               launch, by their width, walls and forcing cells; small ones, to
                                about 256^2, up to 1024 steps in calls of ten or so steps or more; the
                                results are those of single steps bit for bit);
                                for FP16 / BF16 LBM_KERNEL_TILED where it applies, else

@@ -411,14 +411,12 @@ int cluster_steps(const lbm_handle* h, int left) {
     const bool kbc = h->p.collision == LBM_COLLISION_KBC, costly = h->faces || kbc;
     if (warp_rows > (costly ? 3 : 4) || left < (costly ? (warp_rows < 3 ? 6 : 16) : 2 * warp_rows + 2)) return 1;
     // A step ends with its slowest warp.  Forcing cells run a function of their own, in memory, for the whole row: with
-    // 1 % of them BGK ran 0.87 to 1.4 times as fast as single steps at 128^2, 0.6 to 0.9 at 192^2, 0.44 to 0.6 at 256^2
-    // (all of them 0.75, 0.45 and 0.32), KBC 0.7 to 1.2, 0.5 and so down; only BGK on 64^2, with four rows to a block,
-    // gains (1.0 to 1.9).  Moving walls through the lattice: 1.4 to 2.8 to 128^2, KBC at 192^2 0.8.  Four rows to a warp
-    // gain while plain ones are among them (a cavity's walls: 40 % of the rows): with walls everywhere 0.7 to 0.96.
+    // 1 % of them BGK ran 1.2 to 1.7 times as fast as single steps at 128^2 (alone 0.87 to 1.4), 0.8 to 0.9 at 192^2, 0.65 to
+    // 0.75 at 256^2, KBC 1.2 to 1.5 at 64^2 (alone 0.85 to 1.45), 1.0 to 1.3 at 128^2 (0.7 to 1.2), 0.6 at 192^2.  Moving walls through the
+    // lattice: 1.3 and more, but 0.9 to 1.05 at 256^2 (alone 0.7) and, with KBC, 1.04 to 1.15 at 192^2 (0.8).
     const RowCounts& n = h->rows;
-    if (n.forced > 16 && (kbc || cluster_rows(h) * windows > 4)) return 1;
-    if (kbc && warp_rows >= 3 && n.rare > 2ull * windows + 48) return 1;
-    if (warp_rows >= 4 && 10 * n.mixed > 6ull * windows * (unsigned)h->ny) return 1;
+    if (n.forced > 16 && (warp_rows > 1 || (kbc && cluster_rows(h) * windows > 4))) return 1;
+    if (n.rare > 2ull * windows + 48 && (warp_rows >= 4 || (kbc && warp_rows >= 3))) return 1;
     int ready = 0;
     const cudaError_t e = h->p.collision == LBM_COLLISION_KBC ? cluster_ready<LBM_COLLISION_KBC>(h->device, &ready)
                                                               : cluster_ready<LBM_COLLISION_BGK>(h->device, &ready);

@@ -113,47 +113,46 @@ bool has_fused_form(const lbm_handle* h) {
 // latency of a row: 1000 x 700 ran 10.4 us a step in single steps and 11.1 fused (600 x 375 6.3 and 7.0).
 constexpr size_t FUSED_CELLS = 800000, FUSED_WALLS = 850000;
 
-// Whether T fused steps are faster than T single ones.  Time of single steps over that of fused ones, measured over
-// widths of 64 to 60,000 columns and 0.8 to 8 million cells, two steps a launch / three:
-//   * BGK in a periodic box 1.15 to 1.55 / 1.3 to 2.1 from 0.8 million cells on.  Walls and faces sit in the first and the
-//     last window, which then hold up a short pass: cavities 0.87 to 1.1 / 0.87 to 1.1 at 0.82 million, 1.07 to 1.2 at 1.25;
-//     channels 0.87 to 1.0 at 0.82, 0.97 to 1.1 / 1.0 to 1.1 at 1.25 million.  KBC, whose rows take longer, the same
-//     0.3 million cells later (cavities 0.83 to 1.0 at 0.82 million, 1.0 to 1.25 at 1.6).
-//   * The reference's rules, whose walls are stored through memory: boxes 0.72 to 0.92 / 0.84 to 1.06 at 0.82 million, 0.97
-//     to 1.1 / 1.14 to 1.3 at 1.6, with a forcing column 0.66 to 0.76 / 0.74 to 0.85, 0.8 to 1.0 / 0.9 to 1.1 at 1.6 and
-//     1.0 to 1.2 / 1.1 to 1.35 at 2.8 million.
-//   * Columns: a window stores 60.  64 wide: 0.73 / 0.68 (channel), 121: 0.66, 181: 0.75; with three quarters of the lanes
-//     filled, faces counted as 1.3 windows more, no case above these sizes is slower than 0.97 (0.8 for two steps of the
-//     reference's rules: 240 wide, with a forcing column, 0.87).
-//   * Rows of less than 24 cells of height: 0.7 to 0.8 at 1.25 million cells.
+// Whether fused steps are faster than single ones.  Time of single steps over that of fused ones, two steps a launch /
+// three, with three lattices on three streams and with one alone:
+//   * 420 to 5000 columns, 0.82 million cells.  Periodic BGK 1.5 / 1.7, alone 1.15 / 1.3; cavity 1.45 / 1.6, alone
+//     1.0 / 1.0; channel 1.4 / 1.5, alone 0.95 / 0.95.  KBC 1.35 / 1.3, 1.25 / 1.2 and 1.2 / 1.1, alone 1.1, 0.95 and 0.9.  The
+//     reference's box 1.35 / 1.4, alone 0.8 / 0.9, with a forcing column 1.27 / 1.33, alone 0.7 / 0.8.  At 2 million 1.5 / 2.0,
+//     1.5 / 2.0, 1.5 / 1.9, KBC 1.5 to 1.55, reference 1.5 / 1.75; alone all gain.  (A lattice alone near the line is held
+//     up by its first and last windows, with walls and faces, in a pass too short to hide them.)
+//   * Columns.  A window stores 60, windows with faces cost 1.5 to 2 more, walls up to 0.6; a width off a multiple of four
+//     copies cell by cell (0.75 of the speed, KBC 0.9).  Channels of 64, 100, 121, 150 and 181 columns 0.65 / 0.58,
+//     1.0 / 0.95, 0.63 / 0.62, 0.9 / 0.87 and 0.75 / 0.72, of 240 and 300 1.25 / 1.3 and 1.4 / 1.45.  What is left of a
+//     window, times the gain of a wide lattice, has to reach 1: of 398 lattices above the lines (64 to 5000 columns, 0.8
+//     to 2.8 million cells, three at a time) two are slower than 0.95, at 0.9; of 178 below, seven gain more than 1.2.
+//   * Less than 24 rows with walls: 0.7 to 0.8.
 //   * Forcing cells, and cells beside moving walls, run a function of their own for the whole row: 1 % of such cells
-//     0.9 / 0.57, one in each window 0.75 / 0.62, all 0.54 / 0.46.  A lid is one row of them.  A column of them in 50
-//     windows costs nothing at 9 million cells (1.4 / 1.8), but 0.83 / 0.92 at 2.3 million.
+//     1.0 / 0.5, one in each window 0.8 / 0.6, all 0.55 / 0.45.  A lid is one row of them; a column of them in 25 windows 1.4 /
+//     1.6 (alone 0.83 / 0.92), twice in 17 windows 1.3 / 1.2 (0.8 / 0.7).
 //   * Walls inside the lattice cost single steps more than fused ones: with 10 % of the cells solid, at random, a million
-//     cells gain 1.48 (BGK) and 1.35 (KBC).  In six of ten rows of the windows they lift the lines above for physics
-//     mode, and in one of five they decide below FUSED_WALLS.  (Not all gain so close to the line: single obstacles in
-//     0.7 % of the cells 0.9 to 1.2 / 0.8 to 1.15, narrow lattices and the reference's boxes 0.6 to 0.9.
-//     tests/test_gpu_fused.py counts launches of those.)
-static bool march_pays(const lbm_handle* h, int T) {
+//     cells gain 1.85 / 2.1 (alone 1.5).  So in one of five rows of the windows they decide below FUSED_WALLS.  (Narrow
+//     lattices lose there all the same, 0.6 to 0.9: tests/test_gpu_fused.py counts launches of those.)
+static bool march_pays(const lbm_handle* h) {
     const size_t windows = (size_t)(h->nx + MARCH_OUT - 1) / MARCH_OUT, rows = windows * (size_t)h->ny;
     const RowCounts& n = h->rows;
-    if (n.rare > 2 * windows + 16 && !(h->N >= 8000000 && n.rare <= rows / 32)) return false;
-    if (h->N < FUSED_WALLS) return 5 * n.inner >= rows;
+    if (n.rare > std::max(2 * windows + 16, rows / 16)) return false;
+    if (h->N < FUSED_WALLS && 5 * n.inner >= rows) return true;
+    const bool kbc = h->p.collision == LBM_COLLISION_KBC, reference = h->p.mode == LBM_MODE_REFERENCE;
     const bool faces = n.face >= (size_t)h->ny / 2, walls = n.mixed > 0;
-    const bool reference = h->p.mode == LBM_MODE_REFERENCE;
-    const double filled = (double)h->nx / (MARCH_OUT * ((double)windows + (faces ? 1.3 : 0.0)));
-    if (filled < (reference && T == 2 ? 0.8 : 0.75) || (h->ny < 24 && walls)) return false;
-    if (reference) return h->N >= (T == 3 ? (faces ? 1950000u : 1550000u) : (faces ? 2750000u : 1950000u));
-    if ((!walls && !faces) || 10 * n.inner >= 6 * rows) return true;
-    return h->N >= (h->p.collision == LBM_COLLISION_KBC ? 1550000u : (faces ? 1300000u : 1200000u));
+    if (h->ny < 24 && walls) return false;
+    const double more = faces ? (kbc ? 2.0 : 1.5) : (walls ? (kbc || reference ? 0.6 : 0.3) : 0.0);
+    const double copies = h->nx % 4 == 0 ? 1.0 : (kbc ? 0.9 : 0.75);
+    const double left = copies * h->nx / (MARCH_OUT * ((double)windows + more));
+    return left >= (kbc ? (faces && h->N < 1200000 ? 0.72 : 0.63) : (reference ? 0.6 : 0.53));
 }
 
 int fused_steps(const lbm_handle* h, int left) {
-    if (!has_fused_form(h) || h->p.macro_every_step || h->countdown > 0 || h->nx < MARCH_W || h->ny < 8 || h->N < FUSED_CELLS)
+    if (left < 2 || !has_fused_form(h) || h->p.macro_every_step || h->countdown > 0 || h->nx < MARCH_W || h->ny < 8 ||
+        h->N < FUSED_CELLS || !march_pays(h))
         return 1;
-    const bool two = even_steps(h) && march_pays(h, 2);
-    if (left >= 3 && !(left == 4 && two) && march_pays(h, 3)) return 3;
-    return left >= 2 && two ? 2 : 1;
+    const bool even = even_steps(h);
+    if (left >= 3 && !(left == 4 && even)) return 3;
+    return even ? 2 : 1;
 }
 
 static FusedLattice fused_lattice(const lbm_handle* h) {

@@ -30,21 +30,24 @@ KBC = dict(collision="kbc")
 
 
 @pytest.mark.parametrize("nx,ny,scene,form,kind,steps,launches", [
-    (1000, 900, "periodic", {}, None, 3, 1), (1000, 1000, "channel", {}, None, 3, 3), (1200, 1150, "channel", {}, None, 3, 1),
-    (1000, 1000, "cavity", {}, None, 2, 2), (300, 4200, "cavity", {}, None, 2, 1), (64, 20000, "cavity", {}, None, 3, 3),
-    (121, 20000, "channel", {}, None, 3, 3), (420, 5000, "channel", {}, None, 4, 2), (60000, 20, "cavity", {}, None, 3, 3),
-    (1200, 1150, "cavity", KBC, None, 3, 3), (1300, 1300, "channel", KBC, None, 3, 1), (1000, 900, "periodic", KBC, None, 2, 1),
-    (1300, 1300, "custom", REF, None, 3, 1), (1300, 1300, "custom", REF, None, 2, 2), (1500, 1400, "custom", REF, None, 2, 1),
-    (1300, 1300, "poiseuille", REF, None, 3, 3), (1500, 1400, "poiseuille", REF, None, 3, 1),
-    (1500, 1400, "poiseuille", REF, None, 4, 2), (1700, 1700, "poiseuille", REF, None, 2, 1), (240, 16000, "poiseuille", REF, None, 2, 2),
-    (1032, 780, "channel", {}, None, 3, 3), (64, 12504, "channel", {}, None, 3, 3), (1032, 780, "channel", {}, "solid", 3, 1), (1000, 1000, "channel", KBC, "solid", 3, 1),
-    (301, 2700, "custom", REF, None, 2, 2),
-    (1500, 1500, "periodic", {}, "column", 3, 3), (3000, 3000, "periodic", {}, "column", 3, 1), (1500, 1500, "periodic", {}, "force", 3, 3),
-    (1500, 1500, "periodic", KBC, "moving", 2, 2), (1500, 1500, "periodic", {}, "solid", 3, 1),
+    # widths, faces and walls
+    (1000, 900, "periodic", {}, None, 3, 1), (1000, 1000, "channel", {}, None, 3, 1), (1000, 1000, "cavity", {}, None, 2, 1),
+    (240, 4000, "channel", {}, None, 3, 1), (421, 2300, "channel", {}, None, 4, 2), (301, 2800, "channel", {}, None, 3, 3),
+    (121, 20000, "channel", {}, None, 3, 3), (100, 9000, "channel", {}, None, 3, 3), (64, 20000, "cavity", {}, None, 3, 3),
+    (100, 9000, "cavity", {}, None, 3, 1), (150, 6000, "periodic", {}, None, 2, 1), (121, 7000, "periodic", {}, None, 2, 2),
+    (60000, 20, "cavity", {}, None, 3, 3), (60000, 20, "periodic", {}, None, 3, 1), (64, 12504, "channel", {}, None, 3, 3),
+    (181, 5000, "periodic", KBC, None, 3, 1), (181, 5000, "cavity", KBC, None, 3, 3), (300, 3000, "cavity", KBC, None, 3, 1),
+    (300, 3000, "channel", KBC, None, 3, 3), (300, 4200, "channel", KBC, None, 3, 1), (420, 2100, "channel", KBC, None, 3, 1),
+    (1300, 700, "custom", REF, None, 2, 1), (301, 2700, "custom", REF, None, 2, 2), (240, 4000, "poiseuille", REF, None, 2, 1),
+    (100, 9000, "poiseuille", REF, None, 2, 2), (1001, 900, "poiseuille", REF, None, 3, 1), (800, 999, "custom", REF, None, 3, 3),
+    # forcing cells, moving walls, walls inside
+    (1000, 1000, "periodic", {}, "column", 3, 3), (1500, 1500, "periodic", {}, "column", 3, 1), (1500, 1500, "periodic", {}, "force", 3, 3),
+    (1500, 1500, "periodic", KBC, "moving", 2, 2), (1500, 1500, "periodic", {}, "solid", 3, 1), (1032, 780, "channel", {}, "solid", 3, 1),
     # small lattices
-    (128, 128, "periodic", {}, None, 20, 1), (128, 128, "periodic", {}, "force", 20, 20), (64, 64, "periodic", {}, "force", 20, 1),
-    (64, 64, "periodic", KBC, "force", 20, 20), (192, 192, "periodic", KBC, "moving", 20, 20),
-    (192, 192, "periodic", {}, "moving", 20, 1), (256, 256, "periodic", {}, "solid", 20, 20), (256, 256, "periodic", {}, None, 20, 1)])
+    (128, 128, "periodic", {}, None, 20, 1), (128, 128, "periodic", {}, "force", 20, 1), (128, 128, "periodic", KBC, "force", 20, 20),
+    (64, 64, "periodic", KBC, "force", 20, 1), (192, 192, "periodic", {}, "force", 20, 20), (192, 192, "periodic", KBC, "moving", 20, 20),
+    (192, 192, "periodic", {}, "moving", 20, 1), (256, 256, "periodic", {}, "moving", 20, 20), (256, 256, "periodic", {}, "solid", 20, 1),
+    (256, 256, "periodic", {}, None, 20, 1)])
 def test_launches(gpu, nx, ny, scene, form, kind, steps, launches):
     from simuverse_gb300 import FluidSimulator
 
